@@ -1,10 +1,11 @@
-// Flash attention forward on the 5th-generation tensor cores (tcgen05 + TMEM + TMA), head dim 128.
+// Flash attention on the 5th-generation tensor cores (tcgen05 + TMEM + TMA).
 //
-// One CTA = 128 query rows of one (sequence, head).  Per 128-key tile:
-//   S = Q K^T        tcgen05.mma 128x128x16 (both operands K-major, TMA-staged with 128-byte swizzle)
+// Forward, head dim 128: attention_fwd_pair.cuh.  Forward, query / key heads of 192 with values of 128 (latent attention): below.
+// One CTA = 128 query rows of one (sequence, head).  Per 64-key tile:
+//   S = Q K^T        tcgen05.mma 128x64x16 (both operands K-major, TMA-staged with 128-byte swizzle)
 //                    into one of two TMEM score buffers, so the next tile's scores are computed
 //                    while this tile's soft-max runs;
-//   soft-max         eight warps, two threads per query row (64 key columns each): tcgen05.ld the
+//   soft-max         eight warps, two threads per query row (32 key columns each): tcgen05.ld the
 //                    row, mask, running max / sum in the exp2 domain, P (bf16) written to shared
 //                    memory in the UMMA K-major swizzled layout, O rescaled in TMEM (tcgen05.ld /
 //                    tcgen05.st) only when a row maximum moved by more than 2^8;
@@ -12,16 +13,15 @@
 // Warp roles (320 threads): warps 0-7 soft-max / epilogue (TMEM lane quarter = warp id % 4), warp 8
 // TMA producer, warp 9 TMEM allocation + MMA issue.  Causal masking is bottom-right aligned when the
 // key sequence is longer than the query sequence, as in the mma.sync kernel of attention.cu,
-// which stays the fallback (other head sizes, backward).
+// which stays the fallback (other head sizes).
 //
 // Every mbarrier wait is bounded; on expiry the kernel records a code in the status word, skips the
 // rest, frees TMEM and returns.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
-#include <cstdlib>
-
 #include "head_tail.cuh"
+#include "packed_f32.cuh"
 #include "tcgen05_utils.cuh"
 
 namespace msrl {
@@ -33,15 +33,13 @@ constexpr int BM = 128, D = 128;
 constexpr uint32_t TILE_HALF = 128 * 64 * 2;          // one [128 rows x 64 cols] bf16 swizzled half tile
 constexpr uint32_t TILE_BYTES = 2 * TILE_HALF;         // 32 KiB
 constexpr uint32_t SMEM_Q = 0;
-constexpr uint32_t TMEM_COLS = 512;                    // backward kernels
-// nqk: 64-column halves of a query / key head (values have two)
-constexpr uint32_t fwd_smem_bytes(int bn, int nqk) {
-  return nqk * TILE_HALF + 2u * (nqk + 2u) * (bn * 64 * 2) + 128u * bn * 2;
-}
+constexpr uint32_t TMEM_COLS = 512;                    // all of it: one block to an SM
+constexpr int BN = 64, NQK = 3;                        // 192-wide heads: keys per tile, 64-column parts of a query / key head
+constexpr uint32_t FWD_SMEM = NQK * TILE_HALF + 2u * (NQK + 2u) * (BN * 64 * 2) + 128u * BN * 2;
 constexpr int OUT_PITCH = 144;
 constexpr int SOFTMAX_WARPS = 8, TMA_WARP = 8, MMA_WARP = 9, THREADS = 320;
 
-enum { ERR_SMEM = 10, ERR_Q = 11, ERR_K = 12, ERR_V = 13, ERR_S = 14, ERR_P = 15, ERR_PV = 16, ERR_EMPTY = 17 };
+enum { ERR_Q = 11, ERR_K = 12, ERR_V = 13, ERR_S = 14, ERR_P = 15, ERR_PV = 16, ERR_EMPTY = 17 };
 
 struct Params {
   __nv_bfloat16* o;
@@ -66,13 +64,9 @@ __device__ __forceinline__ int head_col(int col0, int gs, int hpg, int hs, int h
   return col0 + (h / hpg) * gs + (h % hpg) * hs;
 }
 
-// BN = keys per tile.  128: one CTA per SM (192 KiB of shared memory, 512 TMEM columns).  64: two
-// CTAs per SM (112 KiB, 256 columns each), so that one CTA's soft-max, prologue and epilogue overlap
-// the other's tensor work.  NQK = 64-column halves of a query / key head: 2, or 3 for the 192-wide heads of latent
-// attention (128 unrotated + 64 rotated entries, values 128), then one CTA per SM.  CAP: soft-capped scores; the cap is
-// monotone, so running maxima are those of the raw scores.
-template <int BN, int NQK, bool CAP>
-__global__ void __launch_bounds__(THREADS, BN == 128 || NQK == 3 ? 1 : 2)
+// CAP: soft-capped scores; the cap is monotone, so running maxima are those of the raw scores.
+template <bool CAP>
+__global__ void __launch_bounds__(THREADS, 1)
 fa_fwd_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ Params p) {
   extern __shared__ unsigned char smem_raw[];
@@ -82,7 +76,7 @@ fa_fwd_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   __shared__ uint32_t tmem_slot;
   constexpr uint32_t KV_HALF = BN * 64 * 2, KV_BYTES = 2 * KV_HALF, K_BYTES = NQK * KV_HALF;
   constexpr uint32_t SMEM_K = NQK * TILE_HALF, SMEM_V = SMEM_K + 2 * K_BYTES, SMEM_P = SMEM_V + 2 * KV_BYTES;
-  constexpr uint32_t TMEM_COLS = BN == 128 ? 512 : 256;      // S0 [0,BN) S1 [BN,2BN) O [2BN, 2BN+128)
+  constexpr uint32_t TMEM_COLS = 256;                        // S0 [0,BN) S1 [BN,2BN) O [2BN, 2BN+128)
   constexpr int HALF = BN / 2, NCH = HALF / 32;              // key columns per soft-max thread
 
   const int b = blockIdx.z, h = blockIdx.y, mt = blockIdx.x;
@@ -98,16 +92,6 @@ fa_fwd_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const int t0 = p.window > 0 ? max(m0 + off - p.window + 1, 0) / BN : 0;
   const int n_tiles = max((max(kmax, 0) + BN - 1) / BN - t0, 0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  {
-    // the tiles must fit behind the 1024-byte alignment of the dynamic segment (the launch leaves
-    // less than a full KiB of slack when two CTAs share an SM)
-    uint32_t dyn;
-    asm volatile("mov.u32 %0, %%dynamic_smem_size;\n" : "=r"(dyn));
-    if ((uint32_t)(smem - smem_raw) + fwd_smem_bytes(BN, NQK) > dyn) {
-      if (threadIdx.x == 0) atomicCAS(p.error, 0, ERR_SMEM);
-      return;
-    }
-  }
   float (*l_part)[BM] = reinterpret_cast<float (*)[BM]>(smem + SMEM_P);   // used after the last P V product
 
   if (threadIdx.x == 0) {
@@ -382,6 +366,14 @@ fa_fwd_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
   }
 }
+
+}  // namespace fa5
+}  // namespace msrl
+
+#include "attention_fwd_pair.cuh"
+
+namespace msrl {
+namespace fa5 {
 
 // =====================================================================================================
 // Backward.  Two kernels, as in attention.cu (no atomics, bit-reproducible):
@@ -917,12 +909,7 @@ MSRL_API int msrl_flash_attn_varlen_fwd_tcgen05(const void* q, const void* k, co
     const long long* l = lay + 4 * i;
     if (l[0] % 8 != 0 || l[1] % 8 != 0 || l[3] % 8 != 0 || l[2] <= 0) return (int)cudaErrorNotSupported;
   }
-  static int bn = 0;
-  if (bn == 0) {
-    const char* e = getenv("MSRL_ATTN_KEY_TILE");
-    bn = (e != nullptr && atoi(e) == 128) ? 128 : 64;
-  }
-  const int nqk = D / 64, kt = nqk == 3 ? 64 : bn;       // 192: only 64-key tiles fit
+  const int kt = D == 192 ? fa5::BN : 128;
   CUtensorMap mq, mk, mv;
   if (!fa5_make_map(&mq, q, Tq, fa5_width(nh, lay[1], lay[2], lay[3], D), lay[0]) ||
       !fa5_make_map(&mk, k, Tk, fa5_width(nkv, lay[5], lay[6], lay[7], D), lay[4], kt) ||
@@ -946,19 +933,30 @@ MSRL_API int msrl_flash_attn_varlen_fwd_tcgen05(const void* q, const void* k, co
   p.k_col0 = 0; p.k_group_stride = (int)lay[5]; p.k_hpg = (int)lay[6]; p.k_head_stride = (int)lay[7];
   p.v_col0 = 0; p.v_group_stride = (int)lay[9]; p.v_hpg = (int)lay[10]; p.v_head_stride = (int)lay[11];
   p.error = error;
-  static bool attr_set[2][2] = {{false, false}, {false, false}};
   const bool capped = softcap > 0.f;
-  const int smem = (int)fa5::fwd_smem_bytes(kt, nqk) + (kt == 64 && nqk == 2 ? 896 : 1024);   // 64, 2: two CTAs in 228 KiB
-  auto* kernel = nqk == 3 ? (capped ? fa5::fa_fwd_tcgen05_kernel<64, 3, true> : fa5::fa_fwd_tcgen05_kernel<64, 3, false>)
-                 : bn == 128 ? (capped ? fa5::fa_fwd_tcgen05_kernel<128, 2, true> : fa5::fa_fwd_tcgen05_kernel<128, 2, false>)
-                             : (capped ? fa5::fa_fwd_tcgen05_kernel<64, 2, true> : fa5::fa_fwd_tcgen05_kernel<64, 2, false>);
-  if (!attr_set[nqk - 2][capped]) {
+  static bool attr_set[2][2] = {{false, false}, {false, false}};
+  const int wide = D == 192, smem = (int)(wide ? fa5::FWD_SMEM : fa5::PAIR_SMEM) + 1024;
+  const void* kernel = wide ? (capped ? (const void*)fa5::fa_fwd_tcgen05_kernel<true> : (const void*)fa5::fa_fwd_tcgen05_kernel<false>)
+                            : (capped ? (const void*)fa5::fa_fwd_pair_kernel<true> : (const void*)fa5::fa_fwd_pair_kernel<false>);
+  if (!attr_set[wide][capped]) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
-    attr_set[nqk - 2][capped] = true;
+    attr_set[wide][capped] = true;
   }
-  dim3 grid((max_q + fa5::BM - 1) / fa5::BM, nh, batch);
-  kernel<<<grid, fa5::THREADS, smem, st>>>(mq, mk, mv, p);
+  const long long tiles = (max_q + fa5::BM - 1) / fa5::BM;
+  if (wide) {
+    dim3 grid((unsigned)tiles, nh, batch);
+    auto* k = capped ? fa5::fa_fwd_tcgen05_kernel<true> : fa5::fa_fwd_tcgen05_kernel<false>;
+    k<<<grid, fa5::THREADS, smem, st>>>(mq, mk, mv, p);
+  } else {
+    // One query tile to a block while all of them fit the machine at once: a block alone with its tile has the exponential units
+    // to itself (about 2300 cycles a key tile, against 2500 for both tiles of a pair).
+    const int width = tiles * nh * batch <= sm_count() ? 1 : 2;
+    const long long groups = (tiles * (nh / nkv) + width - 1) / width, blocks = groups * nkv * batch;
+    if (blocks > 0x7fffffffLL) return (int)cudaErrorNotSupported;
+    auto* k = capped ? fa5::fa_fwd_pair_kernel<true> : fa5::fa_fwd_pair_kernel<false>;
+    k<<<(unsigned)blocks, fa5::PAIR_THREADS, smem, st>>>(mq, mk, mv, p, batch, (int)groups, width);
+  }
   return (int)cudaGetLastError();
 }
 

@@ -172,6 +172,41 @@ def test_flash_attention_fwd_tcgen05(nh, nkv, interleaved, causal, monkeypatch):
 
 
 @pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("nh,nkv,ql,kl", [
+    (3, 1, [127, 128, 129, 1], [127, 128, 129, 1]),              # few tiles: one query tile to a block
+    (3, 1, [64], [64 + 2000]),                                   # a short portion behind many cached keys
+    (6, 2, [255, 256, 257, 385, 1, 900], [255, 256, 257, 385, 1, 900]),   # pairs across row tiles (three heads a group), odd counts
+    (2, 2, [1300] * 9, [1300, 1301, 1427, 1428, 1429, 3000, 2000, 1400, 1556]),   # pairs of row tiles, ends inside and on a tile
+    (16, 2, [300, 700, 128], [100, 701, 1]),                     # rows that see nothing when causal
+])
+def test_flash_attention_fwd_query_tile_pairs(nh, nkv, ql, kl, causal, monkeypatch):
+    """Blocks of one and of two query tiles at the borders of tiles and pairs, against the mma.sync kernel and, where every row
+    sees a key, the fp32 formulation.  Scores of several tens (q scaled by 6) move the running maximum."""
+    from mindspeed_rl_b200 import ops
+    from mindspeed_rl_b200.ops.layouts import QKVLayout
+    torch.manual_seed(13)
+    lay = QKVLayout(nh, nkv, 128, True)
+    cu_q, cu_k = (torch.tensor([0] + list(torch.tensor(x).cumsum(0)), dtype=torch.int32) for x in (ql, kl))
+    tk = int(cu_k[-1])
+    qkv = (6.0 * torch.randn(int(cu_q[-1]), lay.width, device=DEV)).bfloat16()
+    k, v = (torch.randn(tk, nkv, 128, device=DEV).bfloat16() for _ in range(2))
+    runs = []
+    for on in "10":
+        monkeypatch.setenv("MSRL_ATTN_TCGEN05", on)
+        runs.append(ops.attn_varlen_fwd(qkv, lay, cu_q.to(DEV), max(ql), causal=causal, kv=(k, v), cu_seqlens_k=cu_k.to(DEV)))
+    G.check_status(torch.device("cuda", torch.cuda.current_device()), "tcgen05 attention")
+    (out, lse), (out_m, lse_m) = runs
+    # P and the output are rounded to bf16 (2^-9 each) over values of order one; the two kernels round P against different
+    # running maxima
+    torch.testing.assert_close(out.float(), out_m.float(), rtol=2e-2, atol=2e-2)
+    torch.testing.assert_close(lse, lse_m, rtol=1e-4, atol=1e-3)
+    if not causal or all(b >= a for a, b in zip(ql, kl)):
+        out_r, lse_r = ops.attn_varlen_fwd(qkv.cpu(), lay, cu_q, max(ql), causal=causal, kv=(k.cpu(), v.cpu()), cu_seqlens_k=cu_k)
+        torch.testing.assert_close(out.float().cpu(), out_r.float(), rtol=2e-2, atol=2e-2)
+        torch.testing.assert_close(lse.cpu(), lse_r, rtol=1e-4, atol=1e-3)
+
+
+@pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("nh,nkv,interleaved", [(4, 2, True), (7, 1, False)])
 def test_flash_attention_bwd_tcgen05(nh, nkv, interleaved, causal, monkeypatch):
     """tcgen05 backward (dQ kernel, dK/dV kernel, delta) against autograd through the fp32
