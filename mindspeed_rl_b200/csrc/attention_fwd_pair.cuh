@@ -14,8 +14,8 @@
 // What bounds it: 16384 exponentials and 1024 tensor-core cycles per tile of 128 x 128 (both units are full at about the same
 // rate on an SM), and the soft-max of one tile plus its own two products in a row.  Before: 64-key tiles, whose 128 x 64 products
 // are bound by shared-memory reads, with P through shared memory and each score read twice from TMEM.  Causal, 28 heads over 4:
-one sequence of 22528, 7361 and 2879 tokens each 6261 -> 3273 us (653 -> 1248 TFLOP/s), 1280 + 3072 + 1863 + 2201 tokens
-334 -> 186 us, eight of 1024 184 -> 127 us.
+// one sequence of 22528, 7361 and 2879 tokens each 6261 -> 3273 us (653 -> 1248 TFLOP/s), 1280 + 3072 + 1863 + 2201 tokens
+// 334 -> 186 us, eight of 1024 184 -> 127 us.
 #pragma once
 
 namespace msrl {
