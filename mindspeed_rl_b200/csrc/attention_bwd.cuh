@@ -8,19 +8,25 @@
 // through shared memory.  The 128 x 128 products read their operands from shared memory at just the rate of the tensor cores
 // (the 128 x 64 ones of smaller tiles are bound by those reads), the ones with A in TMEM at half of it.  Eight soft-max warps:
 // two threads to a TMEM lane, 64 columns each; a thread's P lies in the first 32 columns of its own scores, so that none is
-// overwritten before its owner has read it.
+// overwritten before its owner has read it.  (Sixteen warps with 32 columns each: the same.)
 //
-// Bound by: 2048 (dK/dV) and 1536 (dQ) tensor-core cycles per pair of tiles beside 1024 cycles of exponentials.
+// Bound by: 2048 (dK/dV) and 1536 (dQ) tensor-core cycles per pair of tiles beside 1024 cycles of exponentials, at the clock the
+// power limit leaves (1.62 GHz; the tensor pipe is busy 72 % of the time in dK/dV).  Both kernels and delta, causal, 28 heads over
+// 4, before (64-key tiles, P and dS through shared memory) and now: 22528 + 7361 + 2879 tokens 15617 -> 12400 us, 1280 + 3072 +
+// 1863 + 2201 tokens 836 -> 553 us, eight of 1024 483 -> 360 us.
 #pragma once
 
 namespace msrl {
 namespace fa5 {
 
-constexpr int BWD_THREADS = 384, BWD_TMA = 8, BWD_MMA = 9;       // warps 0-7 soft-max, 8 TMA, 9 MMA
-// two resident tiles (K, V or Q, dO) and two stages of the two that stream by
-constexpr uint32_t BWD_A = 0, BWD_B = TILE_BYTES, BWD_X = 2 * TILE_BYTES, BWD_Y = 4 * TILE_BYTES, BWD_SMEM = 6 * TILE_BYTES;
+constexpr int BWD_WARPS = 8, BWD_TMA = 8, BWD_MMA = 9, BWD_THREADS = 384;      // warps 0-7 soft-max, 8 TMA, 9 MMA
+constexpr int NC = 512 / BWD_WARPS;                    // columns of a soft-max thread
+// Two resident tiles (K, V or Q, dO) and stages of the two that stream by.
+constexpr uint32_t BWD_A = 0, BWD_B = TILE_BYTES, BWD_X = 2 * TILE_BYTES, DKDV_Y = 4 * TILE_BYTES, DKDV_SMEM = 6 * TILE_BYTES;
+// dQ: three stages of K, which the last product of a step frees and the next but one step reads first (with two, every step waited
+// for its K: 666 us against 528 for one sequence of 8192, 28 heads over 4).
+constexpr uint32_t DQ_Y = 5 * TILE_BYTES, DQ_SMEM = 7 * TILE_BYTES;
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr int MAX_SPLIT = 8;
 
 struct BwdParams {
   const __nv_bfloat16* o;
@@ -105,11 +111,11 @@ __device__ __forceinline__ void tile_product(uint32_t tmem_c, uint32_t a, uint32
     umma(tmem_c, desc_sw128(a + (kk >> 2) * TILE_HALF + (kk & 3) * 32, 16, 1024),
          desc_sw128(b + (kk >> 2) * TILE_HALF + (kk & 3) * 32, 16, 1024), id, kk > 0 ? 1u : 0u);
 }
-// tmem_c (+)= A B for 16 of the 128 inner rows: A bf16 in TMEM (two groups of 64, each in the first half of its 64 columns),
+// tmem_c (+)= A B for 16 of the 128 inner rows: A bf16 in TMEM (NC to a soft-max thread, in the first half of its columns),
 // B [128 inner rows, 128] MN-major in shared memory
 __device__ __forceinline__ void tmem_step(uint32_t tmem_c, uint32_t tmem_a, uint32_t b, int kk, bool add) {
   constexpr uint32_t id = idesc_bf16(BM, D, true);
-  umma_ts(tmem_c, tmem_a + (kk >> 2) * 64 + (kk & 3) * 8, desc_sw128(b + kk * 2048, TILE_HALF, 1024), id, add ? 1u : 0u);
+  umma_ts(tmem_c, tmem_a + kk * 16 / NC * NC + kk * 16 % NC / 2, desc_sw128(b + kk * 2048, TILE_HALF, 1024), id, add ? 1u : 0u);
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float2 v) {
@@ -151,11 +157,11 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       mbar_init(&q_empty[i], 1);
       mbar_init(&do_full[i], 1);
       mbar_init(&do_empty[i], 1);
-      mbar_init(&p_part[i], 8);
+      mbar_init(&p_part[i], BWD_WARPS);
     }
     mbar_init(&s_full, 1);
     mbar_init(&dp_full, 1);
-    mbar_init(&ds_ready, 8);
+    mbar_init(&ds_ready, BWD_WARPS);
     mbar_init(&done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -209,7 +215,7 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (ok) {
           mbar_expect_tx(&do_full[st], TILE_BYTES);
           for (int i = 0; i < 2; ++i)
-            tma_load_2d(smem + BWD_Y + st * TILE_BYTES + i * TILE_HALF, &map_do, &do_full[st], hq * D + i * 64, q0 + qr);
+            tma_load_2d(smem + DKDV_Y + st * TILE_BYTES + i * TILE_HALF, &map_do, &do_full[st], hq * D + i * 64, q0 + qr);
         }
       }
       ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
@@ -229,7 +235,7 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         ok = ok && mbar_wait(&do_full[n & 1], (n >> 1) & 1, p.error, ERR_Q);
         if (!ok) return;
         fence_after();
-        tile_product(tm_dp, base + BWD_B, base + BWD_Y + (n & 1) * TILE_BYTES);
+        tile_product(tm_dp, base + BWD_B, base + DKDV_Y + (n & 1) * TILE_BYTES);
         commit(&dp_full);
       };
       ok = mbar_wait(&kv_full, 0, p.error, ERR_K);
@@ -237,7 +243,7 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       dprobs(0);
       for (int n = 0; n < n_it && ok; ++n) {
         const int st = n & 1;
-        const uint32_t q_addr = base + BWD_X + st * TILE_BYTES, do_addr = base + BWD_Y + st * TILE_BYTES;
+        const uint32_t q_addr = base + BWD_X + st * TILE_BYTES, do_addr = base + DKDV_Y + st * TILE_BYTES;
         // dV += P^T dO, the first half of each thread's columns as soon as it is there
 #pragma unroll
         for (int part = 0; part < 2; ++part) {
@@ -261,7 +267,7 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       }
       if (ok) commit(&done);
     }
-  } else if (warp < 8) {
+  } else if (warp < BWD_WARPS) {
     const int wg = warp >> 2, quarter = warp & 3;
     const int key = kb + quarter * 32 + lane;
     const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
@@ -301,7 +307,7 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           packed[i] = pack_bf16(a);
           packed[i + 1] = pack_bf16(e);
         }
-        tmem_st16(ts + part * 16, packed);
+        tmem_st_cols(ts + part * 16, packed);
         tmem_wait_st();
         fence_before();
         __syncwarp();
@@ -323,7 +329,7 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           packed[i + 1] =
               pack_bf16(unpack2(mul2(pack2(s[c + 2], s[c + 3]), add2(pack2(dp[c + 2], dp[c + 3]), pack2(d.z, d.w)))));
         }
-        tmem_st16(tdp + part * 16, packed);
+        tmem_st_cols(tdp + part * 16, packed);
       }
       tmem_wait_st();
       fence_before();
@@ -415,7 +421,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  __shared__ uint64_t qdo_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], dp_full, dp_free, ds_ready, done;
+  __shared__ uint64_t qdo_full, k_full[3], k_empty[3], v_full[2], v_empty[2], s_full[2], dp_full, dp_free, ds_ready, done;
   __shared__ uint32_t tmem_slot;
 
   // longest key ranges first
@@ -430,16 +436,18 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
   if (threadIdx.x == 0) {
     mbar_init(&qdo_full, 1);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < 3; ++i) {
       mbar_init(&k_full[i], 1);
       mbar_init(&k_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1);
     }
     mbar_init(&dp_full, 1);
-    mbar_init(&dp_free, 8);
-    mbar_init(&ds_ready, 8);
+    mbar_init(&dp_free, BWD_WARPS);
+    mbar_init(&ds_ready, BWD_WARPS);
     mbar_init(&done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -463,17 +471,15 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       for (int i = 0; i < 2; ++i) tma_load_2d(smem + BWD_A + i * TILE_HALF, &map_q, &qdo_full, qc + i * 64, q0 + m0);
       for (int i = 0; i < 2; ++i) tma_load_2d(smem + BWD_B + i * TILE_HALF, &map_do, &qdo_full, h * D + i * 64, q0 + m0);
       for (int j = 0; j < n_tiles; ++j) {
-        const int st = j & 1;
-        const uint32_t use = j >> 1;
-        // V of a tile is needed once, before its K is free
-        if (use > 0 && !mbar_wait(&v_empty[st], (use - 1) & 1, p.error, ERR_EMPTY)) break;
-        mbar_expect_tx(&v_full[st], TILE_BYTES);
+        const int sk = j % 3, sv = j & 1;
+        if (j >= 3 && !mbar_wait(&k_empty[sk], (j / 3 - 1) & 1, p.error, ERR_EMPTY)) break;
+        mbar_expect_tx(&k_full[sk], TILE_BYTES);
         for (int i = 0; i < 2; ++i)
-          tma_load_2d(smem + BWD_Y + st * TILE_BYTES + i * TILE_HALF, &map_v, &v_full[st], vc + i * 64, k0 + j * 128);
-        if (use > 0 && !mbar_wait(&k_empty[st], (use - 1) & 1, p.error, ERR_EMPTY)) break;
-        mbar_expect_tx(&k_full[st], TILE_BYTES);
+          tma_load_2d(smem + BWD_X + sk * TILE_BYTES + i * TILE_HALF, &map_k, &k_full[sk], kc + i * 64, k0 + j * 128);
+        if (j >= 2 && !mbar_wait(&v_empty[sv], ((j >> 1) - 1) & 1, p.error, ERR_EMPTY)) break;
+        mbar_expect_tx(&v_full[sv], TILE_BYTES);
         for (int i = 0; i < 2; ++i)
-          tma_load_2d(smem + BWD_X + st * TILE_BYTES + i * TILE_HALF, &map_k, &k_full[st], kc + i * 64, k0 + j * 128);
+          tma_load_2d(smem + DQ_Y + sv * TILE_BYTES + i * TILE_HALF, &map_v, &v_full[sv], vc + i * 64, k0 + j * 128);
       }
     }
   } else if (warp == BWD_MMA) {
@@ -481,10 +487,10 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       const uint32_t base = smem_u32(smem);
       bool ok = mbar_wait(&qdo_full, 0, p.error, ERR_Q);
       auto scores = [&](int j) {                           // over dS of tile j - 2, which the product with K has read
-        ok = ok && mbar_wait(&k_full[j & 1], (j >> 1) & 1, p.error, ERR_K);
+        ok = ok && mbar_wait(&k_full[j % 3], (j / 3) & 1, p.error, ERR_K);
         if (!ok) return;
         fence_after();
-        tile_product(tmem + (j & 1) * 128, base + BWD_A, base + BWD_X + (j & 1) * TILE_BYTES);
+        tile_product(tmem + (j & 1) * 128, base + BWD_A, base + BWD_X + j % 3 * TILE_BYTES);
         commit(&s_full[j & 1]);
       };
       auto dprobs = [&](int j) {
@@ -492,7 +498,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         if (ok && j > 0) ok = mbar_wait(&dp_free, (j - 1) & 1, p.error, ERR_S);
         if (!ok) return;
         fence_after();
-        tile_product(tm_dp, base + BWD_B, base + BWD_Y + (j & 1) * TILE_BYTES);
+        tile_product(tm_dp, base + BWD_B, base + DQ_Y + (j & 1) * TILE_BYTES);
         commit(&dp_full);
         commit(&v_empty[j & 1]);
       };
@@ -506,14 +512,14 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         ok = ok && mbar_wait(&ds_ready, j & 1, p.error, ERR_P);
         if (!ok) break;
         fence_after();
-        const uint32_t k_addr = base + BWD_X + (j & 1) * TILE_BYTES;
+        const uint32_t k_addr = base + BWD_X + j % 3 * TILE_BYTES;
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) tmem_step(tm_dq, tmem + (j & 1) * 128, k_addr, kk, j > 0 || kk > 0);   // dQ += dS K
-        commit(&k_empty[j & 1]);
+        commit(&k_empty[j % 3]);
       }
       if (ok) commit(&done);
     }
-  } else if (warp < 8) {
+  } else if (warp < BWD_WARPS) {
     const int wg = warp >> 2, quarter = warp & 3;
     const int grow = m0 + quarter * 32 + lane;
     const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
@@ -524,16 +530,16 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     const f2 scale2 = pack2(p.scale_log2, p.scale_log2), nl2 = pack2(nl, nl), nd2 = pack2(nd, nd);
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
-      const uint32_t ts = tmem + (j & 1) * 128 + lanes + wg * 64;
+      const uint32_t ts = tmem + (j & 1) * 128 + lanes + wg * NC;
       ok = mbar_wait_warp(&s_full[j & 1], (j >> 1) & 1, p.error, ERR_S);
       if (!ok) break;
       fence_after();
-      float s[64];
-      tmem_ld_cols<64>(ts, s);
+      float s[NC];
+      tmem_ld_cols<NC>(ts, s);
       const bool masked = j * 128 + 128 > klen || (p.causal && j * 128 + 127 > m0 + off);
-      const int limit = masked ? min(klen, p.causal ? grow + off + 1 : klen) - j * 128 - wg * 64 : 64;   // valid columns
+      const int limit = masked ? min(klen, p.causal ? grow + off + 1 : klen) - j * 128 - wg * NC : NC;   // valid columns
 #pragma unroll
-      for (int c = 0; c < 64; c += 2) {
+      for (int c = 0; c < NC; c += 2) {
         float2 a = unpack2(fma2(pack2(s[c], s[c + 1]), scale2, nl2));
         a = make_float2(ex2(a.x), ex2(a.y));
         if (masked) {
@@ -545,20 +551,20 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       ok = mbar_wait_warp(&dp_full, j & 1, p.error, ERR_S);
       if (!ok) break;
       fence_after();
-      float dp[64];
-      tmem_ld_cols<64>(tm_dp + lanes + wg * 64, dp);
+      float dp[NC];
+      tmem_ld_cols<NC>(tm_dp + lanes + wg * NC, dp);
       fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&dp_free);
 #pragma unroll
-      for (int part = 0; part < 2; ++part) {
+      for (int c = 0; c < NC; c += 32) {
         uint32_t packed[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const int c = part * 32 + 2 * i;
-          packed[i] = pack_bf16(unpack2(mul2(pack2(s[c], s[c + 1]), add2(pack2(dp[c], dp[c + 1]), nd2))));
+          const int e = c + 2 * i;
+          packed[i] = pack_bf16(unpack2(mul2(pack2(s[e], s[e + 1]), add2(pack2(dp[e], dp[e + 1]), nd2))));
         }
-        tmem_st16(ts + part * 16, packed);
+        tmem_st_cols(ts + c / 2, packed);
       }
       tmem_wait_st();
       fence_before();
@@ -566,7 +572,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (lane == 0) mbar_arrive(&ds_ready);
     }
     if (ok && n_tiles > 0) ok = mbar_wait_warp(&done, 0, p.error, ERR_PV);
-    if (ok) {
+    if (ok && wg < 2) {
       if (n_tiles > 0) fence_after();
       const int qc = head_col(0, p.q_group_stride, p.q_hpg, p.q_head_stride, h);
       store_half_tile(tm_dq + lanes + wg * 64, p.scale, n_tiles == 0, smem + warp * (32 * OUT_PITCH), lane,

@@ -252,7 +252,7 @@ fa_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             const __nv_bfloat162 h2 = __floats2bfloat162_rn(v.x, v.y);
             packed[i] = *reinterpret_cast<const uint32_t*>(&h2);
           }
-          tmem_st16(tm_s + c * 16, packed);
+          tmem_st_cols(tm_s + c * 16, packed);
           if (c & 1) {
             tmem_wait_st();
             fence_before();

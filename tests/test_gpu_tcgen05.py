@@ -232,6 +232,42 @@ def test_flash_attention_bwd_tcgen05(nh, nkv, interleaved, causal, monkeypatch):
     torch.testing.assert_close(dqkv.float(), dqkv_m.float(), rtol=3e-2, atol=5e-2)
 
 
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("nh,nkv,ql,kl", [
+    (3, 1, [127, 128, 129, 1], [127, 128, 129, 1]),              # borders of a tile; odd heads
+    (7, 1, [700], [700]),                                        # key tiles shared by two blocks, odd number of steps
+    (2, 1, [2], [2]),                                            # one step to each of the two blocks
+    (8, 8, [385, 130, 900, 513] * 8, [385, 130, 900, 513] * 8),  # many key tiles: one block each
+    (4, 2, [130, 64, 500], [1500, 64, 257]),                     # more keys than queries, and fewer
+])
+def test_flash_attention_bwd_key_tiles(nh, nkv, ql, kl, causal, monkeypatch):
+    """Backward with one and with two blocks to a key tile, at the borders of 128-row tiles, against the formulas in fp32 with
+    the log-sum-exp of the forward (where rows see no key at all, which the formulas answer with nan, against the mma.sync
+    kernels).  Run twice: the same bits."""
+    from mindspeed_rl_b200 import ops
+    torch.manual_seed(14)
+    cu_q, cu_k = (torch.tensor([0] + list(torch.tensor(x).cumsum(0)), dtype=torch.int32) for x in (ql, kl))
+    tq, tk = int(cu_q[-1]), int(cu_k[-1])
+    q = torch.randn(tq, nh, 128, device=DEV).bfloat16()
+    k, v = (torch.randn(tk, nkv, 128, device=DEV).bfloat16() for _ in range(2))
+    do = torch.randn(tq, nh * 128, device=DEV).bfloat16()
+    out, lse = ops.attn_kv_fwd(q, k, v, cu_q.to(DEV), cu_k.to(DEV), max(ql), causal)
+    got, again = (ops.attn_kv_bwd(do, q, k, v, out, lse, cu_q.to(DEV), cu_k.to(DEV), max(ql), max(kl), causal) for _ in range(2))
+    G.check_status(torch.device("cuda", torch.cuda.current_device()), "tcgen05 attention")
+    if causal and any(a > b for a, b in zip(ql, kl)):
+        monkeypatch.setenv("MSRL_ATTN_TCGEN05", "0")
+        ref = ops.attn_kv_bwd(do, q, k, v, out, lse, cu_q.to(DEV), cu_k.to(DEV), max(ql), max(kl), causal)
+    else:
+        ref = ops.attn_kv_bwd(do.cpu().float(), q.cpu().float(), k.cpu().float(), v.cpu().float(), out.cpu().float(), lse.cpu(),
+                              cu_q, cu_k, max(ql), max(kl), causal)
+    for a, b, c in zip(got, again, ref):
+        assert torch.equal(a, b)
+        a, c = a.float().cpu(), c.float().cpu()
+        # P and dS are rounded to bf16 (2^-9 of each term, averaged over the sum) and so is the result
+        assert ((a - c).norm() / c.norm()).item() < 6e-3
+        torch.testing.assert_close(a, c, rtol=2e-2, atol=2e-2 * c.abs().max().item())
+
+
 @pytest.mark.parametrize("causal", [False, True])
 def test_block_attention_with_separate_kv(causal):
     """The block primitives of ring attention (queries against a separate K/V block, log-sum-exp of the
