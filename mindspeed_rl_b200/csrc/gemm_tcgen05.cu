@@ -4,12 +4,8 @@
 //   4-stage shared-memory ring guarded by full/empty mbarriers;
 // * one elected thread issues tcgen05.mma (cta_group::1, 128x256x16) on UMMA shared-memory
 //   descriptors; tcgen05.commit releases ring slots and finally signals the epilogue;
-// * four epilogue warps read the 128x256 fp32 accumulator out of TMEM with tcgen05.ld and apply
-//   a fused epilogue:
-//     - STORE: convert to bf16 and store C;
-//     - LOGPROB_STATS: LM-head fused with the log-softmax statistics -- every row's running
-//       (max, sum-exp, target logit, sum e^z z) over this tile's 256 vocabulary columns is
-//       written as one 16-byte record; the logits themselves never reach global memory.
+// * four epilogue warps read the 128x256 fp32 accumulator out of TMEM with tcgen05.ld, convert to bf16 and
+//   store C.
 //
 // Every wait on an mbarrier is bounded (wall-clock limit); on expiry the kernel records an error
 // code, skips the remaining work, still frees its TMEM allocation and returns, so the host sees
@@ -58,10 +54,6 @@ constexpr int G_MAX_RANKS = 16;
 constexpr int G_COMM_THREADS = 128;
 constexpr int G_AG_PIECES = 16;      // a 128-row tile is copied as 16 pieces of 8 rows
 constexpr int G_RS_CHUNKS = 16;      // a row tile is reduced as 16 column chunks (spreads the tail over CTAs)
-
-struct RowStat4 {
-  float m, s, zy, spz;
-};
 
 // ---- mbarrier / TMA / tcgen05 wrappers ----------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -169,18 +161,10 @@ constexpr uint32_t make_idesc_bf16(int m, int n) {
          | ((uint32_t)(m >> 4) << 24);  // M / 16
 }
 
-enum Epilogue { EPI_STORE = 0, EPI_LOGPROB_STATS = 1 };
-
 struct GemmParams {
   int M, N, K;
-  // EPI_STORE
   __nv_bfloat16* C;
   long long ldc;
-  // EPI_LOGPROB_STATS
-  const long long* labels;  // [M] global vocabulary ids
-  int vocab_offset;         // first vocabulary id of column 0
-  float inv_temp;
-  RowStat4* stats;          // [num_n_tiles, M]
   int* error;               // device status word (0 = ok)
   // communication-fused variants
   int rank, world;
@@ -252,7 +236,7 @@ __device__ __forceinline__ void tile_coords(int tile, int m_tiles, int n_tiles, 
   }
 }
 
-template <int EPI, int COMM>
+template <int COMM>
 __global__ void __launch_bounds__(COMM == COMM_NONE ? 192 : 192 + G_COMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_a_local, const __grid_constant__ GemmParams p) {
@@ -377,7 +361,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       tcgen05_fence_after();
       const int row = m0 + warp * 32 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(warp * 32) << 16) + buf * G_BN;
-      if (EPI == EPI_STORE) {
+      {
         __nv_bfloat16* cbase = p.C;
         long long ldc = p.ldc, crow = row;
         if (COMM == COMM_RS) {
@@ -432,47 +416,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           __threadfence_system();
           __syncwarp();
           if (lane == 0) red_release_sys_add(p.peer_flag[mt / mt_local] + (mt % mt_local), 1u);
-        }
-      } else {
-        float mx = -INFINITY, s = 0.f, spz = 0.f, zy = 0.f;
-        const long long label = (row < p.M) ? p.labels[row] - p.vocab_offset : -1;
-#pragma unroll 1
-        for (int c = 0; c < G_BN / 32; ++c) {
-          float v[32];
-          tmem_ld32(t_row + c * 32, v);
-          const int col = n0 + c * 32;
-          float cm = -INFINITY;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            // logits take the bf16 rounding the un-fused path would apply before the softmax
-            v[j] = (col + j < p.N) ? __bfloat162float(__float2bfloat16(v[j])) * p.inv_temp : -INFINITY;
-            cm = fmaxf(cm, v[j]);
-          }
-          if (cm > mx) {
-            const float corr = __expf(mx - cm);
-            s *= corr;
-            spz *= corr;
-            mx = cm;
-          }
-          if (mx > -INFINITY) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (col + j < p.N) {
-                const float e = __expf(v[j] - mx);
-                s += e;
-                spz += e * v[j];
-              }
-            }
-          }
-          if (label >= col && label < col + 32 && label < p.N) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (label == col + j) zy = v[j];
-          }
-        }
-        if (row < p.M) {
-          RowStat4 o{mx, s, zy, spz};
-          p.stats[(long long)nt * p.M + row] = o;
         }
       }
       // hand the accumulator back to the MMA warp
@@ -613,7 +556,7 @@ static bool make_map(CUtensorMap* map, const void* base, long long rows, long lo
   return r == CUDA_SUCCESS;
 }
 
-template <int EPI, int COMM = COMM_NONE>
+template <int COMM = COMM_NONE>
 static int launch_gemm(const void* A, long long lda, const void* B, long long ldb, const GemmParams& p,
                        cudaStream_t st, const void* A_local = nullptr, long long lda_local = 0) {
   CUtensorMap ma, mb, ml;
@@ -623,7 +566,7 @@ static int launch_gemm(const void* A, long long lda, const void* B, long long ld
   if (A_local != nullptr && !make_map(&ml, A_local, p.m_local, p.K, lda_local, G_BM))
     return (int)cudaErrorInvalidValue;
   const size_t smem = (size_t)G_STAGES * G_STAGE_BYTES + G_EPI_BYTES + 1024;
-  cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<EPI, COMM>,
+  cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<COMM>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const int tiles = ((p.M + G_BM - 1) / G_BM) * ((p.N + G_BN - 1) / G_BN);
@@ -631,7 +574,7 @@ static int launch_gemm(const void* A, long long lda, const void* B, long long ld
   // work of the whole grid, and every CTA must be resident for the counters to advance.
   const int grid = (COMM != COMM_NONE || tiles >= sm_count()) ? sm_count() : tiles;
   const int threads = COMM == COMM_NONE ? 192 : 192 + G_COMM_THREADS;
-  gemm_tcgen05_kernel<EPI, COMM><<<grid, threads, smem, st>>>(ma, mb, ml, p);
+  gemm_tcgen05_kernel<COMM><<<grid, threads, smem, st>>>(ma, mb, ml, p);
   return (int)cudaGetLastError();
 }
 
@@ -650,26 +593,7 @@ MSRL_API int msrl_gemm_bf16_tn(const void* A, long long lda, const void* B, long
   p.C = (__nv_bfloat16*)C;
   p.ldc = ldc;
   p.error = error;
-  return launch_gemm<EPI_STORE>(A, lda, B, ldb, p, st);
-}
-
-MSRL_API int msrl_lmhead_stats_tiles(int N) { return (N + G_BN - 1) / G_BN; }
-
-// LM head fused with the log-softmax statistics: stats[tile_n, M] records over 256-column tiles
-// of z = (H W^T) * inv_temp; combine them with msrl_logprob_finish(nshard = tiles * shards).
-MSRL_API int msrl_lmhead_stats(const void* H, long long ldh, const void* W, long long ldw,
-                               const long long* labels, int vocab_offset, float inv_temp, void* stats,
-                               int M, int N, int K, int* error, cudaStream_t st) {
-  if (M == 0 || N == 0) return 0;
-  if (K % 8 != 0) return (int)cudaErrorInvalidValue;
-  GemmParams p{};
-  p.M = M; p.N = N; p.K = K;
-  p.labels = labels;
-  p.vocab_offset = vocab_offset;
-  p.inv_temp = inv_temp;
-  p.stats = (RowStat4*)stats;
-  p.error = error;
-  return launch_gemm<EPI_LOGPROB_STATS>(H, ldh, W, ldw, p, st);
+  return launch_gemm(A, lda, B, ldb, p, st);
 }
 
 // ---- communication-fused GEMMs over peer-mapped memory ------------------------------------------
@@ -696,7 +620,7 @@ MSRL_API int msrl_ag_gemm_bf16_tn(void* const* peer_a, long long ld_peer, void* 
   p.tile_ready = tile_ready;
   cudaError_t e = cudaMemsetAsync(tile_ready, 0, sizeof(unsigned int) * (size_t)(p.M / G_BM), st);
   if (e != cudaSuccess) return (int)e;
-  return launch_gemm<EPI_STORE, COMM_AG>(gathered, K, B, ldb, p, st, peer_a[rank], ld_peer);
+  return launch_gemm<COMM_AG>(gathered, K, B, ldb, p, st, peer_a[rank], ld_peer);
 }
 
 MSRL_API int msrl_gemm_rs_tiles(int N) { return (N + G_BN - 1) / G_BN; }
@@ -727,5 +651,5 @@ MSRL_API int msrl_gemm_rs_bf16_tn(const void* A, long long lda, const void* B, l
   p.rs_done = done;
   p.rs_out = (__nv_bfloat16*)out;
   p.ld_out = ld_out;
-  return launch_gemm<EPI_STORE, COMM_RS>(A, lda, B, ldb, p, st);
+  return launch_gemm<COMM_RS>(A, lda, B, ldb, p, st);
 }
