@@ -17,7 +17,7 @@
 //  * operand forms: K-major (rows of K contiguous elements) and MN-major (the matrix stored
 //    transposed, [K, rows]) for A and for B through the UMMA descriptors, so forward (x W^T), data
 //    gradient (dy W) and weight gradient (dy^T x) all read the tensors where they are;
-//  * epilogues: bf16 store (+ bias), accumulate into an fp32 / bf16 C (weight gradients add
+//  * epilogues: bf16 store (+ bias), SwiGLU of the two halves of the first MLP linear, accumulate into an fp32 / bf16 C (weight gradients add
 //    into the flat gradient buffer), or the log-softmax statistics of the LM head, whose logits are never written.
 //
 // Every wait is bounded; on expiry the status word is set, all roles drain and both CTAs still free
@@ -44,7 +44,7 @@ constexpr uint32_t TMEM_COLS = 512;               // two 128 x 256 fp32 accumula
 constexpr int EPI_PITCH = 144;
 constexpr uint32_t EPI_BYTES = 4 * 32 * EPI_PITCH;
 enum { ERR_FULL = 31, ERR_EMPTY = 32, ERR_ACC = 33 };
-enum OutMode { OUT_BF16 = 0, OUT_ACC_F32 = 1, OUT_ACC_BF16 = 2, OUT_PART_F32 = 3, OUT_STATS = 4 };
+enum OutMode { OUT_BF16 = 0, OUT_ACC_F32 = 1, OUT_ACC_BF16 = 2, OUT_PART_F32 = 3, OUT_STATS = 4, OUT_SWIGLU = 5 };
 enum CommMode { COMM_NONE = 0, COMM_AG = 1, COMM_RS = 2 };
 enum { ERR_GATHER = 34, ERR_PEERS = 35 };
 constexpr int MAX_RANKS = 16;
@@ -71,6 +71,9 @@ struct Params {
   long long c_group_stride;
   int k_splits;                // OUT_PART_F32: pieces the reduction is cut into (one work item per tile and piece;
                                // piece s writes its fp32 partial tile into slab s of C, [k_splits, M, ldc])
+  // OUT_SWIGLU: C [M, N] = silu(gate) * up, with B = [gate rows | up rows], N each; a tile is 128 columns of gate (the leader's rows
+  // of B) beside the same columns of up (its partner's), so that both meet in one accumulator row
+  __nv_bfloat16* gate_up;      // [M, 2 N], may be null: the two products as well
   // OUT_STATS
   const long long* labels;     // [M] global vocabulary ids
   int vocab_offset;            // id of column 0
@@ -202,7 +205,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();            // 0: leader (issues the MMAs), 1: its partner
-  const int m_tiles = (p.M + BM - 1) / BM, n_tiles = (p.N + BN - 1) / BN;
+  constexpr int TN = OUT == OUT_SWIGLU ? BN / 2 : BN;      // output columns of a tile
+  const int m_tiles = (p.M + BM - 1) / BM, n_tiles = (p.N + TN - 1) / TN;
   const int tiles_per_group = m_tiles * n_tiles;
   const bool grouped = (OUT == OUT_ACC_F32 || OUT == OUT_ACC_BF16) && COMM == COMM_NONE && p.groups > 0;
   const int total_tiles = tiles_per_group * ((OUT == OUT_PART_F32) ? p.k_splits : (grouped ? p.groups : 1));
@@ -269,7 +273,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         krange(tile, kb0, kb1);
         if (grouped && kb1 <= kb0) continue;
         coords(tile, mt, nt);
-        const int m0 = mt * BM + (int)rank * HM, n0 = nt * BN + (int)rank * HN;
+        const int m0 = mt * BM + (int)rank * HM, n0 = nt * TN + (int)rank * (OUT == OUT_SWIGLU ? p.N : HN);
         const CUtensorMap* amap = &map_a;
         int a_row = m0;
         if (COMM == COMM_AG) {
@@ -368,7 +372,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const uint32_t buf = local & 1;
       int mt, nt;
       coords(tile, mt, nt);
-      const int m0 = mt * BM + (int)rank * HM, n0 = nt * BN;
+      const int m0 = mt * BM + (int)rank * HM, n0 = nt * TN;
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (local >> 1) & 1, p.error, ERR_ACC) &&
                                        (*reinterpret_cast<volatile int*>(p.error) == 0));
       if (!ok) break;
@@ -430,6 +434,53 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             asm volatile("red.release.sys.global.add.u32 [%0], %1;\n" ::"l"(p.peer_flag[mt / mt_local] + unit), "r"(1u)
                          : "memory");
           }
+        }
+      } else if constexpr (OUT == OUT_SWIGLU) {
+        // 64 columns in the warp's patch -> whole 128-byte row segments
+        auto flush = [&](__nv_bfloat16* base, long long ld, int first) {
+          __syncwarp();
+          const int col = first + (lane & 7) * 8;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int r = i * 4 + (lane >> 3);
+            if (m0 + warp * 32 + r < p.M && col < p.N)
+              st8(base + (long long)(m0 + warp * 32 + r) * ld + col, *reinterpret_cast<const bf16x8*>(patch + r * EPI_PITCH + (lane & 7) * 16));
+          }
+          __syncwarp();
+        };
+#pragma unroll 1
+        for (int c = 0; c < TN / 64; ++c) {
+          if (n0 + c * 64 >= p.N) break;
+          if (p.gate_up != nullptr) {
+#pragma unroll 1
+            for (int up = 0; up < 2; ++up) {
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                float v[32];
+                tmem_ld32(t_row + up * TN + c * 64 + h * 32, v);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                  *reinterpret_cast<bf16x8*>(patch + lane * EPI_PITCH + h * 64 + q * 16) = pack8(v + q * 8);
+              }
+              flush(p.gate_up + (long long)up * p.N, 2LL * p.N, n0 + c * 64);
+            }
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            float g[32], u[32];
+            tmem_ld32(t_row + c * 64 + h * 32, g);
+            tmem_ld32(t_row + TN + c * 64 + h * 32, u);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              // both products rounded to bf16 first, as when they go through memory
+              const float gg = __bfloat162float(__float2bfloat16(g[j])), uu = __bfloat162float(__float2bfloat16(u[j]));
+              g[j] = gg / (1.f + __expf(-gg)) * uu;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              *reinterpret_cast<bf16x8*>(patch + lane * EPI_PITCH + h * 64 + q * 16) = pack8(g + q * 8);
+          }
+          flush(reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, n0 + c * 64);
         }
       } else if constexpr (OUT == OUT_STATS) {
         float mx = -INFINITY, s = 0.f, spz = 0.f, zy = 0.f;
@@ -695,7 +746,8 @@ static int launch(const void* A, long long lda, const void* B, long long ldb, co
   CUtensorMap ma, mb, ml;
   // K-major: [rows, K], box 64 k x 128 rows; MN-major: [K, rows], box 64 rows x 64 k
   const bool oka = A_MN ? make_map(&ma, A, p.M, p.K, lda, 64, 64) : make_map(&ma, A, p.K, p.M, lda, BK, HM);
-  const bool okb = B_MN ? make_map(&mb, B, p.N, p.K, ldb, 64, 64) : make_map(&mb, B, p.K, p.N, ldb, BK, HN);
+  const int b_rows = OUT == OUT_SWIGLU ? 2 * p.N : p.N;
+  const bool okb = B_MN ? make_map(&mb, B, b_rows, p.K, ldb, 64, 64) : make_map(&mb, B, p.K, b_rows, ldb, BK, HN);
   if (!oka || !okb) return (int)cudaErrorInvalidValue;
   ml = ma;
   if (A_local != nullptr && !make_map(&ml, A_local, p.K, p.m_local, lda_local, BK, HM)) return (int)cudaErrorInvalidValue;
@@ -714,7 +766,8 @@ static int launch(const void* A, long long lda, const void* B, long long ldb, co
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) n = sm_count() / 2;
     max_clusters = n < sm_count() / 2 ? n : sm_count() / 2;
   }
-  const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) *
+  const int tn = OUT == OUT_SWIGLU ? BN / 2 : BN;
+  const int tiles = ((p.M + BM - 1) / BM) * ((p.N + tn - 1) / tn) *
                     (OUT == OUT_PART_F32 ? p.k_splits : (p.groups > 0 ? p.groups : 1));
   // the fused variants always launch every pair: their comm warps share the copy / reduce work of the
   // whole grid, and every CTA must be resident for the counters to advance
@@ -781,6 +834,24 @@ MSRL_API int msrl_gemm_pair_bf16(const void* A, long long lda, int a_mn, const v
   if (a_mn && b_mn && out_mode == g2::OUT_ACC_F32) return g2::launch<true, true, g2::OUT_ACC_F32>(A, lda, B, ldb, p, st);
   if (a_mn && b_mn && out_mode == g2::OUT_ACC_BF16) return g2::launch<true, true, g2::OUT_ACC_BF16>(A, lda, B, ldb, p, st);
   return (int)cudaErrorInvalidValue;
+}
+
+// act [M, F] = silu(A gate^T) * (A up^T) with W [2 F, K] = [gate | up], and the two products in gate_up [M, 2 F] unless it is
+// null.  Both products are rounded to bf16 before the SwiGLU: the same bits as the plain linear followed by the SwiGLU kernel,
+// whose pass over memory (read 2 F, write F columns a token; without gate_up also the linear's 2 F) this saves.
+MSRL_API int msrl_gemm_pair_swiglu(const void* A, long long lda, const void* W, long long ldw, void* act, void* gate_up,
+                                   int M, int F, int K, int* error, cudaStream_t st) {
+  if (M == 0 || F == 0) return 0;
+  if (K <= 0 || K % 8 != 0 || F % 8 != 0 || F > 0x3fffffff || (reinterpret_cast<uintptr_t>(act) & 15) != 0 ||
+      (reinterpret_cast<uintptr_t>(gate_up) & 15) != 0)
+    return (int)cudaErrorInvalidValue;
+  g2::Params p{};
+  p.M = M; p.N = F; p.K = K;
+  p.C = act;
+  p.ldc = F;
+  p.gate_up = (__nv_bfloat16*)gate_up;
+  p.error = error;
+  return g2::launch<false, false, g2::OUT_SWIGLU>(A, lda, W, ldw, p, st);
 }
 
 MSRL_API int msrl_lmhead_stats_tiles(int N) { return (N + g2::BN - 1) / g2::BN; }

@@ -225,10 +225,12 @@ def layer_forward(layer: TransformerLayer, h: torch.Tensor, meta: PackedMeta, ke
     # residual add fused into the norm: one pass writes h1 = h + proj and its normalised form
     x2, rstd2, h1 = ops.rmsnorm_fwd(proj, layer.pre_mlp_layernorm.weight, eps, residual=h, want_rstd=keep)
     if isinstance(layer.mlp, MLP):
-        gu, x2g = comm.column_linear(x2, layer.mlp.linear_fc1.weight)
         if lora.active(layer.mlp.linear_fc1):
+            gu, x2g = comm.column_linear(x2, layer.mlp.linear_fc1.weight)
             lo["fc1"] = lora.column_fwd(layer.mlp.linear_fc1, x2g, gu)
-        y = ops.swiglu_fwd(gu)
+            y = ops.swiglu_fwd(gu)
+        else:
+            y, gu, x2g = comm.column_linear_swiglu(x2, layer.mlp.linear_fc1.weight, keep)
         mlp_out = comm.row_linear(y, layer.mlp.linear_fc2.weight)
         if lora.active(layer.mlp.linear_fc2):
             lo["fc2"] = lora.row_fwd(layer.mlp.linear_fc2, y, mlp_out, comm)[1]

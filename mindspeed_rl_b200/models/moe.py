@@ -317,8 +317,7 @@ class MoELayer(nn.Module):
         over TP under sequence parallelism (identity otherwise), the row-parallel output is reduce-scattered
         (all-reduced) back."""
         xg = comm.gather_seq(x)
-        gu = _gemm.linear_fwd(xg, self.shared_experts.linear_fc1.weight)
-        act = ops.swiglu_fwd(gu)
+        act, gu = _gemm.linear_swiglu(xg, self.shared_experts.linear_fc1.weight, keep)
         y = comm.reduce_out(_gemm.linear_fwd(act, self.shared_experts.linear_fc2.weight))
         return y, ((xg, gu, act) if keep else None)
 

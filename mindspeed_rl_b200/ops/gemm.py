@@ -154,6 +154,24 @@ def linear_fwd(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = 
     return torch.matmul(x, w.t())
 
 
+def linear_swiglu(x: torch.Tensor, w: torch.Tensor, keep: bool = False
+                  ) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
+    """``(silu(g) * u, gate_up if keep else None)`` with ``gate_up = [g | u] = x [T, K] @ w [2 F, K].T``: the first linear of an MLP
+    and its activation.  Where the CTA-pair kernel takes the linear, one kernel does both, with the same bits."""
+    if (x.is_cuda and x.dim() == 2 and w.shape[0] % 16 == 0 and pair_usable(x, w) and _lib.use_kernels(x, w)
+            and _pair_pays(x.shape[0], w.shape[0])):
+        m, f = x.shape[0], w.shape[0] // 2
+        act = guard.empty(m, f, device=x.device, dtype=torch.bfloat16)
+        gate_up = guard.empty(m, 2 * f, device=x.device, dtype=torch.bfloat16) if keep else None
+        check(_lib.load().msrl_gemm_pair_swiglu(
+            ptr(x), c_ll(x.stride(0)), ptr(w), c_ll(w.stride(0)), ptr(act), ptr(gate_up), c_int(m), c_int(f),
+            c_int(x.shape[1]), ptr(_status_word(x.device)), stream()), "gemm_pair_swiglu")
+        return act, gate_up
+    from .elementwise import swiglu_fwd
+    gate_up = linear_fwd(x, w)
+    return swiglu_fwd(gate_up), (gate_up if keep else None)
+
+
 def linear_f32(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """``x [T, K] @ w [N, K].T`` with a 32-bit result: few output columns (router and gate logits), whatever the
     operands' type."""

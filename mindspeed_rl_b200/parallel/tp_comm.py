@@ -17,7 +17,8 @@ from typing import Optional
 import torch
 import torch.distributed as dist
 
-from ..ops.gemm import linear_dgrad, linear_fwd
+from ..ops.elementwise import swiglu_fwd
+from ..ops.gemm import linear_dgrad, linear_fwd, linear_swiglu
 
 
 class TPComm:
@@ -87,6 +88,14 @@ class TPComm:
         if bias is not None:
             y += bias
         return y, xg
+
+    def column_linear_swiglu(self, x: torch.Tensor, w: torch.Tensor, keep: bool):
+        """``(silu(g) * u, [g | u] if keep else None, gather_seq(x))`` with ``[g | u] = gather_seq(x) @ w.T``."""
+        if self._fused_ok(x) and self.fused.fits_ag(x, w):
+            gate_up, xg = self.fused.ag_gemm(x, w)
+            return swiglu_fwd(gate_up), (gate_up if keep else None), xg
+        xg = self.gather_seq(x)
+        return (*linear_swiglu(xg, w, keep), xg)
 
     def row_linear(self, a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
         """``reduce_out(a @ w.T)``."""

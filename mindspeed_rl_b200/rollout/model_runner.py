@@ -23,7 +23,7 @@ import torch
 from .. import ops
 from ..models.transformer_config import TransformerConfig
 from ..ops import QKVLayout
-from ..ops.gemm import linear_fwd
+from ..ops.gemm import linear_fwd, linear_swiglu
 from ..parallel.tp_comm import NO_TP, TPComm
 from .layer_cache import HybridCache
 from .mixers import StepMeta
@@ -169,7 +169,7 @@ class ModelRunner:
         if lw.moe is not None:
             delta = lw.moe.forward(x, self.comm)
         else:
-            y = ops.swiglu_fwd(linear_fwd(x, lw.gate_up_w))
+            y = linear_swiglu(x, lw.gate_up_w)[0]
             delta = self.comm.all_reduce(linear_fwd(y, lw.down_w))
         return resid, delta
 

@@ -124,10 +124,10 @@ class MoEWeights:
         return self._add_shared(out.to(x.dtype), x, comm, fork)
 
     def _shared_mlp(self, x: torch.Tensor) -> torch.Tensor:
-        from ..ops.gemm import linear_fwd
+        from ..ops.gemm import linear_fwd, linear_swiglu
 
         fc1, fc2 = self.shared
-        return linear_fwd(ops.swiglu_fwd(linear_fwd(x, fc1)), fc2)
+        return linear_fwd(linear_swiglu(x, fc1)[0], fc2)
 
     def _fork_shared(self, x: torch.Tensor):
         """Start the shared experts on a side stream, so that they run beside the routed experts' token

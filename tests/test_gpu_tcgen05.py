@@ -97,6 +97,31 @@ def test_gemm_pair_data_and_weight_gradient_forms(m, n, k):
     G.check_status(DEV)
 
 
+@pytest.mark.parametrize("m,f,k", [(129, 6144, 64), (256, 6200, 200), (300, 6168, 192), (1025, 8, 264), (2000, 1544, 1096)])
+def test_gemm_pair_swiglu(m, f, k):
+    """SwiGLU in the epilogue of the first MLP linear: the bits of the plain kernel followed by the SwiGLU kernel, with widths
+    that end inside a tile of 128 and of 64 columns, and rows that end inside a tile."""
+    from mindspeed_rl_b200 import ops
+    torch.manual_seed(4)
+    x = torch.randn(m, k, device=DEV).bfloat16()
+    w = (0.2 * torch.randn(2 * f, k, device=DEV)).bfloat16()
+    gate_up = G.gemm_pair(x, w)
+    want = ops.swiglu_fwd(gate_up)
+    L = _lib.load()
+    for keep in (False, True):
+        act = torch.full((m, f), 7.0, device=DEV).bfloat16()
+        gu = torch.full((m, 2 * f), 7.0, device=DEV).bfloat16() if keep else None
+        assert L.msrl_gemm_pair_swiglu(ptr(x), c_ll(k), ptr(w), c_ll(k), ptr(act), ptr(gu), c_int(m), c_int(f), c_int(k),
+                                       ptr(G._status_word(x.device)), stream()) == 0
+        G.check_status(DEV)
+        assert torch.equal(act, want)
+        if keep:
+            assert torch.equal(gu, gate_up)
+        got, got_gu = G.linear_swiglu(x, w, keep)
+        assert (got_gu is None) == (not keep)
+        _assert_close(got, torch.nn.functional.silu(gate_up[:, :f].float()) * gate_up[:, f:].float(), k)
+
+
 @pytest.mark.parametrize("t,v,h", [(200, 1000, 256), (513, 5000, 896)])
 def test_lmhead_stats_fused(t, v, h):
     torch.manual_seed(1)
