@@ -373,6 +373,29 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       int mt, nt;
       coords(tile, mt, nt);
       const int m0 = mt * BM + (int)rank * HM, n0 = nt * TN;
+      // Accumulating epilogues: what C holds is fetched 32 columns ahead, the first of them before the wait for the products (an
+      // expert's weight gradient has a handful of k-blocks to a tile, and the loads in their turn took longer than those: the four
+      // weight gradients of an expert layer, 128 experts of 2048 x 768, 16384 tokens, 3052 -> 1783 us).
+      constexpr bool ACC = OUT == OUT_ACC_F32 || OUT == OUT_ACC_BF16;
+      constexpr int CV = OUT == OUT_ACC_F32 ? 8 : 4;          // 16-byte vectors of C a lane has of 32 columns
+      uint4 c_next[ACC ? CV : 1];
+      const long long group_off = grouped ? (long long)(tile / tiles_per_group) * p.c_group_stride : 0;
+      const bool c_vec = (p.ldc & (OUT == OUT_ACC_BF16 ? 7 : 3)) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
+      // vector i of this lane in columns [col0, col0 + 32): row of the warp's 32, address in C
+      auto c_row = [&](int i) { return OUT == OUT_ACC_BF16 ? i * 8 + (lane >> 2) : i * 4 + (lane >> 3); };
+      auto c_at = [&](int col0, int i) {
+        const long long row_off = group_off + (long long)(m0 + warp * 32 + c_row(i)) * p.ldc + col0;
+        return OUT == OUT_ACC_BF16 ? reinterpret_cast<char*>(p.C) + (row_off + (lane & 3) * 8) * 2
+                                   : reinterpret_cast<char*>(p.C) + (row_off + (lane & 7) * 4) * 4;
+      };
+      auto c_fetch = [&](int c) {
+        const int col0 = n0 + c * 32;
+        if (!c_vec || col0 + 32 > p.N) return;
+#pragma unroll
+        for (int i = 0; i < CV; ++i)
+          if (m0 + warp * 32 + c_row(i) < p.M) c_next[i] = *reinterpret_cast<const uint4*>(c_at(col0, i));
+      };
+      if constexpr (ACC) c_fetch(0);
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (local >> 1) & 1, p.error, ERR_ACC) &&
                                        (*reinterpret_cast<volatile int*>(p.error) == 0));
       if (!ok) break;
@@ -524,20 +547,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         // Accumulating epilogues (weight gradients): C += acc through the warp's shared-memory patch, so
         // that the read-modify-write of C moves whole 128-byte (fp32) / 64-byte (bf16) row segments per
         // group of lanes instead of one 16-byte piece per lane and row.  32 columns per step, fp32 staging.
-        const long long crow0 = m0 + warp * 32;
-        const bool f32 = (OUT == OUT_ACC_F32 || OUT == OUT_PART_F32);
+        constexpr bool f32 = OUT != OUT_ACC_BF16;
         // split reduction: this piece's slab of the partial-sum buffer; an empty piece (more pieces than
         // k-blocks) was never multiplied and stores zeros
-        const long long group_off = grouped ? (long long)(tile / tiles_per_group) * p.c_group_stride : 0;
         float* const Cf = reinterpret_cast<float*>(p.C) + group_off +
                           ((OUT == OUT_PART_F32) ? (long long)(tile % k_splits) * p.M * p.ldc : 0);
         const bool empty_piece = (OUT == OUT_PART_F32) && (tile % k_splits) * kb_per >= num_kb;
-        const bool vec_ok = f32 ? ((p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0)
-                                : ((p.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
           const int col0 = n0 + c * 32;
           if (col0 >= p.N) break;
+          uint4 c_old[ACC ? CV : 1];
+          if constexpr (ACC) {
+#pragma unroll
+            for (int i = 0; i < CV; ++i) c_old[i] = c_next[i];
+            if (c + 1 < BN / 32) c_fetch(c + 1);
+          }
           float v[32];
           tmem_ld32(t_row + c * 32, v);
           if (empty_piece) {
@@ -548,46 +573,39 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           for (int q = 0; q < 8; ++q)
             *reinterpret_cast<float4*>(patch + lane * EPI_PITCH + q * 16) = make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
           __syncwarp();
-          if (vec_ok && col0 + 32 <= p.N) {
-            if (f32) {
-              float* C = Cf;
+          if (c_vec && col0 + 32 <= p.N) {
+            if constexpr (OUT == OUT_PART_F32) {
               const int cc = (lane & 7) * 4;                    // 8 lanes x 16 B = one 128-byte row segment
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 const int r = i * 4 + (lane >> 3);
-                if (crow0 + r < p.M) {
-                  float* dst = C + (crow0 + r) * p.ldc + col0 + cc;
-                  const float4 a = *reinterpret_cast<const float4*>(patch + r * EPI_PITCH + cc * 4);
-                  if (OUT == OUT_PART_F32) {
-                    *reinterpret_cast<float4*>(dst) = a;
-                  } else {
-                    float4 o = *reinterpret_cast<const float4*>(dst);
-                    o.x += a.x; o.y += a.y; o.z += a.z; o.w += a.w;
-                    *reinterpret_cast<float4*>(dst) = o;
-                  }
-                }
+                if (m0 + warp * 32 + r < p.M)
+                  *reinterpret_cast<float4*>(Cf + (long long)(m0 + warp * 32 + r) * p.ldc + col0 + cc) =
+                      *reinterpret_cast<const float4*>(patch + r * EPI_PITCH + cc * 4);
               }
             } else {
-              __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C) + group_off;
-              const int cc = (lane & 3) * 8;                    // 4 lanes x 16 B = one 64-byte row segment
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const int r = i * 8 + (lane >> 2);
-                if (crow0 + r < p.M) {
-                  __nv_bfloat16* dst = C + (crow0 + r) * p.ldc + col0 + cc;
+              for (int i = 0; i < CV; ++i) {
+                const int r = c_row(i);
+                if (m0 + warp * 32 + r >= p.M) continue;
+                if constexpr (f32) {
+                  const float4 a = *reinterpret_cast<const float4*>(patch + r * EPI_PITCH + (lane & 7) * 16);
+                  const float4 o = *reinterpret_cast<const float4*>(&c_old[i]);
+                  *reinterpret_cast<float4*>(c_at(col0, i)) = make_float4(o.x + a.x, o.y + a.y, o.z + a.z, o.w + a.w);
+                } else {
                   float f[8];
-                  unpack8(ld8(dst), f);
-                  const float4 a0 = *reinterpret_cast<const float4*>(patch + r * EPI_PITCH + cc * 4);
-                  const float4 a1 = *reinterpret_cast<const float4*>(patch + r * EPI_PITCH + cc * 4 + 16);
+                  unpack8(*reinterpret_cast<const bf16x8*>(&c_old[i]), f);
+                  const float4 a0 = *reinterpret_cast<const float4*>(patch + r * EPI_PITCH + (lane & 3) * 32);
+                  const float4 a1 = *reinterpret_cast<const float4*>(patch + r * EPI_PITCH + (lane & 3) * 32 + 16);
                   f[0] += a0.x; f[1] += a0.y; f[2] += a0.z; f[3] += a0.w;
                   f[4] += a1.x; f[5] += a1.y; f[6] += a1.z; f[7] += a1.w;
-                  st8(dst, pack8(f));
+                  *reinterpret_cast<bf16x8*>(c_at(col0, i)) = pack8(f);
                 }
               }
             }
           } else if (row < p.M) {
             const float* src = reinterpret_cast<const float*>(patch + lane * EPI_PITCH);
-            if (f32) {
+            if constexpr (f32) {
               float* dst = Cf + (long long)row * p.ldc + col0;
               for (int jj = 0; jj < 32 && col0 + jj < p.N; ++jj) dst[jj] = (OUT == OUT_PART_F32) ? src[jj] : dst[jj] + src[jj];
             } else {
