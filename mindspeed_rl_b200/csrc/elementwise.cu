@@ -131,7 +131,7 @@ rmsnorm_fwd_regs_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
                         int H, float eps) {
   __shared__ float red[2][32];
   const int nvec = H >> 3;
-  bf16x8 cur[VPT], cur_res[VPT], nxt[VPT], nxt_res[VPT];
+  bf16x8 cur[VPT], cur_res[VPT], nxt[VPT], nxt_res[VPT], wr[1];
   auto fetch = [&](long long r, bf16x8 (&dst)[VPT], bf16x8 (&dst_res)[VPT]) {
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
@@ -144,6 +144,7 @@ rmsnorm_fwd_regs_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
   };
   long long r = blockIdx.x;
   if (r < rows) fetch(r, cur, cur_res);
+  if constexpr (VPT == 1) wr[0] = ld8(w + (threadIdx.x < nvec ? threadIdx.x : 0) * 8);   // ahead of the sum
   int flip = 0;
   for (; r < rows; r += gridDim.x, flip ^= 1) {
     const long long rn = r + gridDim.x;
@@ -184,7 +185,7 @@ rmsnorm_fwd_regs_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
       const int i = threadIdx.x + j * THREADS;
       if (i < nvec) {
         float wv[8], o[8];
-        unpack8(ld8(w + i * 8), wv);
+        unpack8(VPT == 1 ? wr[0] : ld8(w + i * 8), wv);
 #pragma unroll
         for (int k = 0; k < 8; ++k) o[k] = f[j][k] * rstd * wv[k];
         st8(y + r * H + i * 8, pack8(o));
@@ -417,47 +418,61 @@ __global__ void headnorm_bwd_kernel(__nv_bfloat16* __restrict__ dy_dx,
 // cos_sin table: [max_pos, hd] fp32 = [cos(0..hd/2) | sin(0..hd/2)] per position.
 // sign = +1 forward, -1 backward (the inverse rotation applied to gradients).
 // --------------------------------------------------------------------------------------------
-__global__ void rope_kernel(__nv_bfloat16* __restrict__ q, HeadLayout Lq, int nq,
-                            __nv_bfloat16* __restrict__ k, HeadLayout Lk, int nk,
-                            const int* __restrict__ positions, const float* __restrict__ cos_sin,
-                            long long T, int hd, float sign) {
-  // one thread rotates 4 pairs: (i..i+3, i+hd/2..i+hd/2+3)
-  const int half = hd >> 1;
-  const int per_head = half >> 2;
-  const long long total = T * (long long)(nq + nk) * per_head;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(idx % per_head);
-    const long long th = idx / per_head;
-    const int h = (int)(th % (nq + nk));
-    const long long t = th / (nq + nk);
-    __nv_bfloat16* base = (h < nq) ? q + head_offset(Lq, t, h) : k + head_offset(Lk, t, h - nq);
-    const int pos = positions[t];
-    const float4 cs = *reinterpret_cast<const float4*>(cos_sin + (long long)pos * hd + c * 4);
-    const float4 sn = *reinterpret_cast<const float4*>(cos_sin + (long long)pos * hd + half + c * 4);
-    uint2 lo_raw = *reinterpret_cast<const uint2*>(base + c * 4);
-    uint2 hi_raw = *reinterpret_cast<const uint2*>(base + half + c * 4);
-    __nv_bfloat162* lo = reinterpret_cast<__nv_bfloat162*>(&lo_raw);
-    __nv_bfloat162* hi = reinterpret_cast<__nv_bfloat162*>(&hi_raw);
-    const float cc[4] = {cs.x, cs.y, cs.z, cs.w};
-    const float s4[4] = {sn.x * sign, sn.y * sign, sn.z * sign, sn.w * sign};
-    float a[4], b[4];
-    float2 t0 = __bfloat1622float2(lo[0]), t1 = __bfloat1622float2(lo[1]);
-    float2 u0 = __bfloat1622float2(hi[0]), u1 = __bfloat1622float2(hi[1]);
-    a[0] = t0.x; a[1] = t0.y; a[2] = t1.x; a[3] = t1.y;
-    b[0] = u0.x; b[1] = u0.y; b[2] = u1.x; b[3] = u1.y;
-    float ra[4], rb[4];
+// A block walks tokens; its threads take (head, V pairs) of a token, V = 8 with 16-byte accesses where base and strides allow, else
+// 4.  Bound by reading and writing the heads once; indices in 32 bits and one division a token and thread (16384 tokens, 28 + 4 heads
+// of 128: 60 -> 54 us, 8192 30 -> 23; before: V = 4 and four 64-bit divisions a vector).
+template <int V>
+__global__ void __launch_bounds__(256)
+rope_kernel(__nv_bfloat16* __restrict__ q, HeadLayout Lq, int nq, __nv_bfloat16* __restrict__ k, HeadLayout Lk, int nk,
+            const int* __restrict__ positions, const float* __restrict__ cos_sin, long long T, int hd, float sign, int per_block) {
+  const int half = hd >> 1, per_head = half / V, per_token = (nq + nk) * per_head;
+  // `per_block` tokens at a time share the block where a token has few vectors
+  for (long long t0 = (long long)blockIdx.x * per_block; t0 < T; t0 += (long long)gridDim.x * per_block) {
+    const int n = (int)(T - t0 < per_block ? T - t0 : per_block) * per_token;
+    for (int i = threadIdx.x; i < n; i += 256) {
+      const int dt = i / per_token, r = i - dt * per_token, h = r / per_head, c = (r - h * per_head) * V;
+      const long long t = t0 + dt;
+      __nv_bfloat16* base = ((h < nq) ? q + head_offset(Lq, t, h) : k + head_offset(Lk, t, h - nq)) + c;
+      const float* cs = cos_sin + (long long)positions[t] * hd + c;
+      alignas(16) float cc[V], sn[V];
+      float a[V], b[V];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      ra[j] = a[j] * cc[j] - b[j] * s4[j];
-      rb[j] = b[j] * cc[j] + a[j] * s4[j];
+      for (int j = 0; j < V; j += 4) {
+        *reinterpret_cast<float4*>(cc + j) = *reinterpret_cast<const float4*>(cs + j);
+        *reinterpret_cast<float4*>(sn + j) = *reinterpret_cast<const float4*>(cs + half + j);
+      }
+      alignas(16) __nv_bfloat162 lo[V / 2], hi[V / 2];
+      if constexpr (V == 8) {
+        *reinterpret_cast<uint4*>(lo) = *reinterpret_cast<const uint4*>(base);
+        *reinterpret_cast<uint4*>(hi) = *reinterpret_cast<const uint4*>(base + half);
+      } else {
+        *reinterpret_cast<uint2*>(lo) = *reinterpret_cast<const uint2*>(base);
+        *reinterpret_cast<uint2*>(hi) = *reinterpret_cast<const uint2*>(base + half);
+      }
+#pragma unroll
+      for (int j = 0; j < V / 2; ++j) {
+        const float2 x = __bfloat1622float2(lo[j]), y = __bfloat1622float2(hi[j]);
+        a[2 * j] = x.x, a[2 * j + 1] = x.y, b[2 * j] = y.x, b[2 * j + 1] = y.y;
+      }
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        const float s = sn[j] * sign, u = a[j] * cc[j] - b[j] * s;
+        b[j] = b[j] * cc[j] + a[j] * s;
+        a[j] = u;
+      }
+#pragma unroll
+      for (int j = 0; j < V / 2; ++j) {
+        lo[j] = __floats2bfloat162_rn(a[2 * j], a[2 * j + 1]);
+        hi[j] = __floats2bfloat162_rn(b[2 * j], b[2 * j + 1]);
+      }
+      if constexpr (V == 8) {
+        *reinterpret_cast<uint4*>(base) = *reinterpret_cast<const uint4*>(lo);
+        *reinterpret_cast<uint4*>(base + half) = *reinterpret_cast<const uint4*>(hi);
+      } else {
+        *reinterpret_cast<uint2*>(base) = *reinterpret_cast<const uint2*>(lo);
+        *reinterpret_cast<uint2*>(base + half) = *reinterpret_cast<const uint2*>(hi);
+      }
     }
-    lo[0] = __floats2bfloat162_rn(ra[0], ra[1]);
-    lo[1] = __floats2bfloat162_rn(ra[2], ra[3]);
-    hi[0] = __floats2bfloat162_rn(rb[0], rb[1]);
-    hi[1] = __floats2bfloat162_rn(rb[2], rb[3]);
-    *reinterpret_cast<uint2*>(base + c * 4) = lo_raw;
-    *reinterpret_cast<uint2*>(base + half + c * 4) = hi_raw;
   }
 }
 
@@ -605,7 +620,13 @@ MSRL_API int msrl_rmsnorm_fwd(const void* x, const void* res, const void* w, voi
     // one wave of persistent blocks: four 128-thread (two 256-thread) blocks fit the registers of an SM
     const long long cap = (long long)sm_count() * (H <= 128 * 4 * 8 ? 4 : 2);
     const unsigned blocks = (unsigned)(rows < cap ? rows : cap);
-    if (H <= 128 * 4 * 8)
+    // Up to two rows to an SM a row takes its latency: one vector a thread and the weights ahead of the sum (3584 wide, residual: 1
+    // row 3.0 -> 2.4 us, 48 x 2048 2.7 -> 2.2, 256 rows 3.75 -> 3.66; 500 rows 4.5 -> 5.7, which stay with four vectors).
+    if (H <= 512 * 8 && rows <= 2LL * sm_count())
+      rmsnorm_fwd_regs_kernel<512, 1><<<blocks, 512, 0, st>>>(
+          (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w,
+          (__nv_bfloat16*)y, (__nv_bfloat16*)sum_out, rstd, rows, H, eps);
+    else if (H <= 128 * 4 * 8)
       rmsnorm_fwd_regs_kernel<128, 4><<<blocks, 128, 0, st>>>(
           (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w,
           (__nv_bfloat16*)y, (__nv_bfloat16*)sum_out, rstd, rows, H, eps);
@@ -702,9 +723,19 @@ MSRL_API int msrl_rope(void* q, long long q_stride_t, int q_group_stride, int q_
   if (hd % 8 != 0) return (int)cudaErrorInvalidValue;
   HeadLayout Lq{q_stride_t, q_group_stride, q_hpg, q_head_stride};
   HeadLayout Lk{k_stride_t, k_group_stride, k_hpg > 0 ? k_hpg : 1, k_head_stride};
-  const long long total = T * (long long)(nq + nk) * (hd / 8);
-  rope_kernel<<<grid_for(total, 256), 256, 0, st>>>((__nv_bfloat16*)q, Lq, nq, (__nv_bfloat16*)k,
-                                                    Lk, nk, positions, cos_sin, T, hd, sign);
+  const bool wide = hd % 16 == 0 && ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15) == 0 &&
+                    (q_stride_t | k_stride_t | q_group_stride | k_group_stride | q_head_stride | k_head_stride) % 8 == 0;
+  const int per_token = (nq + nk) * (hd / (wide ? 16 : 8));
+  if (per_token == 0) return 0;
+  const int per_block = per_token < 256 ? 256 / per_token : 1;
+  const long long want = ceil_div(T, per_block), cap = (long long)sm_count() * 8;
+  const unsigned blocks = (unsigned)(want < cap ? want : cap);
+  if (wide)
+    rope_kernel<8><<<blocks, 256, 0, st>>>((__nv_bfloat16*)q, Lq, nq, (__nv_bfloat16*)k, Lk, nk, positions, cos_sin, T, hd, sign,
+                                           per_block);
+  else
+    rope_kernel<4><<<blocks, 256, 0, st>>>((__nv_bfloat16*)q, Lq, nq, (__nv_bfloat16*)k, Lk, nk, positions, cos_sin, T, hd, sign,
+                                           per_block);
   MSRL_LAUNCH_CHECK();
 }
 
