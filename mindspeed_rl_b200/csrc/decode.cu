@@ -101,13 +101,23 @@ constexpr int kGroupMax = 8;
 
 // Query / key heads of DK and value heads of DV entries.  A CTA serves 16 query heads of a KV group; larger groups take
 // several (blockIdx.y = KV head x head tile).
+// Of every 64 keys a warp takes sixteen, through a ring of its own: no block barrier between the first key and the last, and the
+// loads of ST - 1 chunks in flight behind the one being multiplied.  Cache slots are looked up a chunk ahead.  Bound by reading K
+// and V, and by what a block costs besides (msrl_paged_decode_nsplit).  With block-wide stages, two of them, heads of 128: 48 sequences
+// of 701 to 3700 keys over 4 KV heads 60 us, 48 now (4.5 TB/s); 256 of 1500 145, now 136 (5.8 TB/s).
+template <int DK, int DV>
+constexpr int decode_stages() { return DK + DV > 256 ? 2 : 3; }
+template <int DK, int DV>
+constexpr size_t decode_smem() {
+  return (size_t)(16 * (DK + 8) + decode_stages<DK, DV>() * 64 * (DK + 8 + DV + 8)) * sizeof(__nv_bfloat16);
+}
 template <int DK, int DV>
 __global__ void __launch_bounds__(128) paged_decode_kernel(const DecodeParams p) {
-  constexpr int CH = 64, LD = DK + 8, LDV = DV + 8, THREADS = 128;
+  constexpr int CH = 64, LD = DK + 8, LDV = DV + 8, THREADS = 128, ST = decode_stages<DK, DV>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem_raw);  // 16 x LD
-  __nv_bfloat16* sK = sQ + 16 * LD;                                 // 2 x CH x LD
-  __nv_bfloat16* sV = sK + 2 * CH * LD;                             // 2 x CH x LDV
+  __nv_bfloat16* sK = sQ + 16 * LD;                                 // 4 warps x ST x 16 x LD
+  __nv_bfloat16* sV = sK + ST * CH * LD;                            // 4 warps x ST x 16 x LDV
 
   const int group = p.nh / p.nkv, tiles = (group + 15) / 16;
   const int b = blockIdx.x, hk = blockIdx.y / tiles, sp = blockIdx.z;
@@ -125,6 +135,14 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const DecodeParams p)
   const int kend = min(ctx, kbeg + per_split);
   const int n_chunks = (kend > kbeg) ? (kend - kbeg + CH - 1) / CH : 0;
 
+  if (n_chunks == 0 && p.slot_total > 1) {                  // a piece without keys: the merge passes it over
+    if (threadIdx.x < rep) {
+      float* ml = p.part_ml + (((long long)b * p.nh + h0 + threadIdx.x) * p.slot_total + p.slot_base + sp) * 2;
+      ml[0] = -INFINITY;
+      ml[1] = 0.f;
+    }
+    return;
+  }
   // Q rows: `rep` heads of this KV group; rows >= rep are zero
   for (int i = threadIdx.x; i < 16 * (DK / 8); i += THREADS) {
     const int r = i / (DK / 8), c = i % (DK / 8);
@@ -132,30 +150,37 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const DecodeParams p)
     const __nv_bfloat16* src = p.q + head_offset(p.Lq, b, h0 + (ok ? r : 0)) + c * 8;
     cp_async16(sQ + r * LD + c * 8, src, ok);
   }
-  const int* bt = p.block_tables + (long long)b * p.max_blocks;
-  auto issue = [&](int chunk, int stage) {
-    const int base = kbeg + chunk * CH;
-    constexpr int VEC = (DK > DV ? DK : DV) / 8;
-    for (int i = threadIdx.x; i < CH * VEC; i += THREADS) {
-      const int r = i / VEC, c = i % VEC;
-      const int key = base + r;
-      const bool ok = key < kend;
-      const int kk = ok ? key : kbeg;
-      int blk, off;
-      if (p.block_shift >= 0) {
-        blk = __ldg(bt + (kk >> p.block_shift));
-        off = kk & (p.block_size - 1);
-      } else {
-        blk = __ldg(bt + kk / p.block_size);
-        off = kk % p.block_size;
-      }
-      const long long row = ((long long)blk * p.block_size + off) * p.nkv + hk;
-      if (DK >= DV || c < DK / 8) cp_async16(sK + (stage * CH + r) * LD + c * 8, p.k_cache + row * DK + c * 8, ok);
-      if (DV >= DK || c < DV / 8) cp_async16(sV + (stage * CH + r) * LDV + c * 8, p.v_cache + row * DV + c * 8, ok);
-    }
-  };
-  if (n_chunks > 0) issue(0, 0);
   cp_async_commit();
+  const int* bt = p.block_tables + (long long)b * p.max_blocks;
+  __nv_bfloat16* const wK = sK + warp * ST * 16 * LD;
+  __nv_bfloat16* const wV = sV + warp * ST * 16 * LDV;
+  // cache slot of this lane's key (lane % 16) of a chunk
+  auto slot_of = [&](int chunk) {
+    const int key = kbeg + chunk * CH + warp * 16 + (lane & 15);
+    const int kk = key < kend ? key : kbeg;
+    if (kk >= ctx) return 0;                                // a split without keys: nothing is read
+    return p.block_shift >= 0 ? (__ldg(bt + (kk >> p.block_shift)) << p.block_shift) + (kk & (p.block_size - 1))
+                              : __ldg(bt + kk / p.block_size) * p.block_size + kk % p.block_size;
+  };
+  int slot = slot_of(0);
+  auto issue = [&](int chunk) {
+    if (chunk < n_chunks) {
+      constexpr int VEC = (DK > DV ? DK : DV) / 8;
+      const int base = kbeg + chunk * CH + warp * 16, stage = chunk % ST;
+#pragma unroll
+      for (int i = 0; i < 16 * VEC / 32; ++i) {
+        const int r = (i * 32 + lane) / VEC, c = (i * 32 + lane) % VEC;
+        const bool ok = base + r < kend;
+        const long long row = (long long)__shfl_sync(0xffffffffu, slot, r) * p.nkv + hk;
+        if (DK >= DV || c < DK / 8) cp_async16(wK + (stage * 16 + r) * LD + c * 8, p.k_cache + row * DK + c * 8, ok);
+        if (DV >= DK || c < DV / 8) cp_async16(wV + (stage * 16 + r) * LDV + c * 8, p.v_cache + row * DV + c * 8, ok);
+      }
+      slot = slot_of(chunk + 1);
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int i = 0; i < ST - 1; ++i) issue(i);
 
   float o_acc[DV / 8][4];
 #pragma unroll
@@ -164,18 +189,14 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const DecodeParams p)
     for (int j = 0; j < 4; ++j) o_acc[i][j] = 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 
+  cp_async_wait<ST - 1>();                                  // the query rows, which all warps share
+  __syncthreads();
   for (int ch = 0; ch < n_chunks; ++ch) {
-    const int st = ch & 1;
-    if (ch + 1 < n_chunks) {
-      issue(ch + 1, st ^ 1);
-      cp_async_commit();
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const __nv_bfloat16* tK = sK + (st * CH + warp * 16) * LD;  // this warp's 16 keys
-    const __nv_bfloat16* tV = sV + (st * CH + warp * 16) * LDV;
+    issue(ch + ST - 1);                                     // over the chunk before, which the whole warp has read
+    cp_async_wait<ST - 1>();
+    __syncwarp();
+    const __nv_bfloat16* tK = wK + ch % ST * 16 * LD;
+    const __nv_bfloat16* tV = wV + ch % ST * 16 * LDV;
     float s[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
 #pragma unroll
     for (int kk = 0; kk < DK / 16; ++kk) {
@@ -247,32 +268,32 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const DecodeParams p)
       mma_16816(o_acc[2 * dp], a, bfr[0], bfr[1]);
       mma_16816(o_acc[2 * dp + 1], a, bfr[2], bfr[3]);
     }
-    __syncthreads();
+    __syncwarp();
   }
   cp_async_wait<0>();
   __syncthreads();
 
-  // merge the 4 warps through shared memory (re-using the K/V stages)
+  // merge the 4 warps through shared memory (re-using the K/V stages), the rows that are heads only
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
     l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
   }
-  float* sO = reinterpret_cast<float*>(sK);        // [4][16][DV]
-  float* sM = sO + 4 * 16 * DV;                     // [4][16]
+  constexpr int LDO = DV + 8;                       // eight rows of float2 without bank conflicts
+  float* sO = reinterpret_cast<float*>(sK);        // [4][16][LDO]
+  float* sM = sO + 4 * 16 * LDO;                    // [4][16]
   float* sL = sM + 4 * 16;                         // [4][16]
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int row = frow + r * 8;
+    if (row >= rep) break;
     if ((lane & 3) == 0) {
       sM[warp * 16 + row] = m_run[r];
       sL[warp * 16 + row] = l_run[r];
     }
 #pragma unroll
-    for (int dt = 0; dt < DV / 8; ++dt) {
-      sO[(warp * 16 + row) * DV + dt * 8 + fcol] = o_acc[dt][2 * r];
-      sO[(warp * 16 + row) * DV + dt * 8 + fcol + 1] = o_acc[dt][2 * r + 1];
-    }
+    for (int dt = 0; dt < DV / 8; ++dt)
+      *reinterpret_cast<float2*>(sO + (warp * 16 + row) * LDO + dt * 8 + fcol) = make_float2(o_acc[dt][2 * r], o_acc[dt][2 * r + 1]);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < rep * DV; i += THREADS) {
@@ -286,7 +307,7 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const DecodeParams p)
     for (int w = 0; w < 4; ++w) {
       const float c = exp2f(sM[w * 16 + r] - mu);
       l += sL[w * 16 + r] * c;
-      o += sO[(w * 16 + r) * DV + d] * c;
+      o += sO[(w * 16 + r) * LDO + d] * c;
     }
     const int h = h0 + r;
     if (p.slot_total == 1) {
@@ -536,7 +557,8 @@ __global__ void __launch_bounds__(128) paged_decode_merge_kernel(const DecodePar
   const float* src = p.part_o + gw * ns * D + lane * V;
 #pragma unroll 4
   for (int s = mine; s < ns; s += wph) {
-    const float c = exp2f(ml[2 * s] - mu);
+    const float ms = ml[2 * s], c = exp2f(ms - mu);
+    if (ms == -INFINITY) continue;                          // no keys: part_o may not have been written
     float v[V];
     if constexpr (V == 4) {
       const float4 x = *reinterpret_cast<const float4*>(src + (long long)s * D);
@@ -905,18 +927,19 @@ MSRL_API int msrl_kv_cache_gather(const void* k_cache, const void* v_cache, cons
 }
 
 // Scratch requirement (floats) for a given problem: part_o = B*nh*nsplit*D, part_ml = B*nh*nsplit*2.
+// Pieces of a sequence's keys.  A block costs about 2.5 us before its first and behind its last key (two are resident on an SM), the
+// longest sequence about a third of the 0.012 us that each of its keys takes a block alone, a merge 3 us; at least 256 keys to a
+// piece.  Kernel alone, heads of 128, 4096 keys at most: 48 sequences of 701 to 3700 keys, 4 KV heads, 1 / 2 / 3 / 4 / 8 / 16 pieces:
+// 66 / 53 / 48 / 47 / 49 / 57 us; 256 of 1 to 1024: 60 / 68 / 68 / 74; 8 of 500 to 2000: 28 / 16 / 12 / 10 / 9 / 10; 1 of 2924: 40
+// alone, 6 in 16.  (Pieces that filled whole waves, the rule before: 8, 2, 8 and 16.)
 MSRL_API int msrl_paged_decode_nsplit(int B, int nkv, int max_ctx) {
-  // Three CTAs of this kernel are resident per SM (shared memory); pick the smallest split count
-  // that fills the machine and wastes under ~10% of the last wave, keeping >= 256 keys per split.
-  const double slots = 3.0 * sm_count();
-  int ns = 1;
-  while (ns < 32 && (max_ctx + 2 * ns - 1) / (2 * ns) >= 256) {
-    const double waves = B * (double)nkv * ns / slots;
-    const double eff = waves / ceil(waves);
-    if (waves >= 1.0 && eff >= 0.9) break;
-    ns *= 2;
+  int best = 1;
+  double best_cost = 1e30;
+  for (int ns = 1; ns <= 32 && (ns == 1 || max_ctx >= 256 * ns); ++ns) {
+    const double cost = 2.5 * ns * B * (double)nkv / (2.0 * sm_count()) + 0.0042 * max_ctx / ns + (ns > 1 ? 3.0 : 0.0);
+    if (cost < best_cost) best = ns, best_cost = cost;
   }
-  return ns;
+  return best;
 }
 
 // tcgen05 form of the shared-prefix pass (decode_prefix_tcgen05.cu)
@@ -967,9 +990,6 @@ static int launch_paged_decode(const void* q, const long long* q_layout4, const 
   p.nsplit = nsplit;
   p.scale_log2 = kLog2eD / sqrtf((float)D);
   const int LD = D + 8;
-  size_t smem = (size_t)(16 + 4 * 64) * LD * sizeof(__nv_bfloat16);
-  const size_t merge_smem = (size_t)(4 * 16 * D + 2 * 4 * 16) * sizeof(float) + 16 * LD * sizeof(__nv_bfloat16);
-  if (merge_smem > smem) smem = merge_smem;
   dim3 grid(B, nkv, nsplit);
   cudaError_t e;
   bool prefix_done = false;
@@ -997,13 +1017,13 @@ static int launch_paged_decode(const void* q, const long long* q_layout4, const 
     if (e != cudaSuccess) return (int)e;
   }
   if (D == 128) {
-    e = cudaFuncSetAttribute(paged_decode_kernel<128, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(paged_decode_kernel<128, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_smem<128, 128>());
     if (e != cudaSuccess) return (int)e;
-    paged_decode_kernel<128, 128><<<grid, 128, smem, st>>>(p);
+    paged_decode_kernel<128, 128><<<grid, 128, decode_smem<128, 128>(), st>>>(p);
   } else {
-    e = cudaFuncSetAttribute(paged_decode_kernel<64, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(paged_decode_kernel<64, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_smem<64, 64>());
     if (e != cudaSuccess) return (int)e;
-    paged_decode_kernel<64, 64><<<grid, 128, smem, st>>>(p);
+    paged_decode_kernel<64, 64><<<grid, 128, decode_smem<64, 64>(), st>>>(p);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
@@ -1026,7 +1046,7 @@ MSRL_API int msrl_paged_decode(const void* q, const long long* q_layout4, const 
 
 template <int DK, int DV>
 static int launch_window_decode(const DecodeParams& p, int B, cudaStream_t st) {
-  constexpr size_t smem = (size_t)(16 * (DK + 8) + 128 * (DK + 8) + 128 * (DV + 8)) * sizeof(__nv_bfloat16);
+  constexpr size_t smem = decode_smem<DK, DV>();
   const cudaError_t e = cudaFuncSetAttribute(paged_decode_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const int tiles = (p.nh / p.nkv + 15) / 16;

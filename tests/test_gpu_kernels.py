@@ -180,6 +180,24 @@ def test_paged_decode_and_cache(nh, nkv, hd, bs):
     assert torch.equal(kg.cpu(), kgr) and torch.equal(vg.cpu(), vgr)
 
 
+@pytest.mark.parametrize("nh,nkv,hd,bs", [(28, 4, 128, 16), (16, 1, 128, 24), (8, 8, 64, 16)])
+@pytest.mark.parametrize("lens", [[1, 15, 16, 17, 64, 65, 129, 1025, 2900], [2900], [191, 192, 193] * 20, [700] * 200])
+def test_paged_decode_pieces(nh, nkv, hd, bs, lens):
+    """Lengths around a warp's sixteen keys and a chunk of 64, in one piece and in many, some of them without keys (a sequence much
+    shorter than the longest that the launch allows for)."""
+    torch.manual_seed(6)
+    lay = QKVLayout(nh, nkv, hd, True)
+    b, maxb = len(lens), (max(lens) + bs - 1) // bs
+    kc, vc = (torch.randn(b * maxb, bs, nkv, hd, device=DEV).bfloat16() for _ in range(2))
+    bt = torch.randperm(b * maxb, device=DEV).to(torch.int32).view(b, maxb)
+    ctx = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    qkv = torch.randn(b, lay.width, device=DEV).bfloat16()
+    ops.paged_decode_attention(10 * qkv, lay, kc, vc, bt, ctx, 4096)        # scratch holds another call's partial results
+    out = ops.paged_decode_attention(qkv, lay, kc, vc, bt, ctx, 4096)
+    ref = ops.paged_decode_attention(qkv.cpu(), lay, kc.cpu(), vc.cpu(), bt.cpu(), ctx.cpu(), 4096)
+    close(out, ref, 2e-2, 2e-2, "out")
+
+
 @pytest.mark.parametrize("nh,nkv,hd,bs,n_samples,prompt", [(28, 4, 128, 16, 8, 200), (8, 2, 64, 16, 5, 70),
                                                            (16, 16, 128, 32, 8, 33), (28, 4, 128, 16, 8, 1100),
                                                            (8, 2, 64, 24, 5, 100)])
