@@ -340,10 +340,14 @@ class MoELayer(nn.Module):
         e, h, f = self.num_local, c.hidden_size, c.moe_ffn_hidden_size
         w1, w2 = self._w1().reshape(h, e * 2 * f), self._w2().reshape(e * f, h)
         plan = K.moe_plan(top_idx, e)
-        xp = K.moe_permute(x, plan)
-        gu = K.grouped_gemm(xp, plan, w1, True, 2 * f, 0, 2 * f)
-        act = ops.swiglu_fwd(gu)
-        y = K.grouped_gemm(act, plan, w2, True, 0, f, h)
+        # weight gradients sum over whole tiles: a forward that a backward follows has its pad rows computed (zero)
+        xp = K.moe_permute(x, plan, zero_pads=keep)
+        if keep:
+            gu = K.grouped_gemm(xp, plan, w1, True, 2 * f, 0, 2 * f)
+            act = ops.swiglu_fwd(gu)
+        else:
+            act = K.grouped_gemm(xp, plan, w1, True, 2 * f, 0, f, pads=False, glu=True)
+        y = K.grouped_gemm(act, plan, w2, True, 0, f, h, pads=keep)
         out = K.moe_combine(y, plan, top_p.detach())
         shared_ctx = None
         if self.shared_experts is not None:

@@ -109,13 +109,14 @@ def route_softmax_top(logits: torch.Tensor, correction: torch.Tensor, top: int) 
     return idx, s.gather(1, idx)
 
 
-def moe_permute(x: torch.Tensor, plan: MoePlan, w: Optional[torch.Tensor] = None) -> torch.Tensor:
+def moe_permute(x: torch.Tensor, plan: MoePlan, w: Optional[torch.Tensor] = None, zero_pads: bool = True) -> torch.Tensor:
     """``x [T, H]`` -> expert-grouped ``[max_rows, H]`` (row of slot (t, j) = ``w[t, j] * x[t]``);
-    pad rows of used segments are zero, rows past the last segment are not touched."""
+    pad rows of used segments are zero (undefined without ``zero_pads``: only for consumers that leave them out), rows past
+    the last segment are not touched."""
     t, h = x.shape
     if x.dtype == torch.float32 and x.is_cuda and w is None and h % 4 == 0:
         # rows are only moved: an fp32 row is a bf16 row of twice the length
-        return moe_permute(x.contiguous().view(torch.bfloat16), plan).view(torch.float32)
+        return moe_permute(x.contiguous().view(torch.bfloat16), plan, zero_pads=zero_pads).view(torch.float32)
     if x.dtype == torch.float32 and _lib.use_kernels(x):
         x = x.contiguous()
         xp = guard.empty(plan.max_rows, h, dtype=x.dtype, device=x.device)
@@ -130,7 +131,7 @@ def moe_permute(x: torch.Tensor, plan: MoePlan, w: Optional[torch.Tensor] = None
         wf = None if w is None else w.reshape(-1).float().contiguous()
         check(_lib.load().msrl_moe_permute(ptr(x), c_ll(h), ptr(plan.pos), ptr(wf), c_int(t), c_int(plan.k), c_int(h),
                                            c_int(plan.num_experts), ptr(plan.counts), ptr(plan.offsets), ptr(xp),
-                                           c_ll(h), stream()), "moe_permute")
+                                           c_ll(h), c_int(int(zero_pads)), stream()), "moe_permute")
         return xp
     # CPU, or rows the kernel cannot move; slots without a row meet in one behind the last
     xp = torch.zeros(plan.max_rows + 1, h, dtype=x.dtype, device=x.device)
@@ -200,12 +201,15 @@ def grouped_wgrad_(grad: torch.Tensor, group_stride: int, ldc: int, a: torch.Ten
 
 
 def grouped_gemm(a: torch.Tensor, plan: MoePlan, b2d: torch.Tensor, b_mn_major: bool, ex: int, ey: int,
-                 n: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                 n: int, out: Optional[torch.Tensor] = None, pads: bool = True, glu: bool = False) -> torch.Tensor:
     """``c[r] = a[r] @ B_e`` for the rows of expert e.  ``b2d`` is a 2-D contiguous view of all
     experts' weights; expert e's operand starts at ``b2d[e*ey, e*ex]`` and is ``[K, n]`` when
     ``b_mn_major`` else ``[n, K]`` (used transposed).  Rows of ``c`` outside used tiles are
-    undefined; pad rows inside used tiles are the product of zero rows."""
+    undefined; pad rows inside used tiles are the product of zero rows, or without ``pads`` neither read nor written.
+    ``glu`` (MN-major only): ``B_e`` is ``[K, 2 n]`` and ``c = silu(a @ B_e[:, :n]) * (a @ B_e[:, n:])``, both products rounded to
+    ``a``'s type first."""
     rows, k = a.shape
+    assert b_mn_major or not glu
     if _lib.use_kernels(a, b2d):
         from .gemm import _status_word
         assert a.is_contiguous() and b2d.is_contiguous() and rows == plan.max_rows
@@ -214,10 +218,15 @@ def grouped_gemm(a: torch.Tensor, plan: MoePlan, b2d: torch.Tensor, b_mn_major: 
         rc = _lib.load().msrl_moe_grouped_gemm(
             ptr(a), c_ll(k), ptr(b2d), c_ll(b2d.shape[0]), c_ll(b2d.shape[1]), c_ll(b2d.shape[1]),
             c_int(1 if b_mn_major else 0), c_int(ex), c_int(ey), ptr(c), c_ll(n), ptr(plan.tile_expert),
-            c_int(rows // PAD), c_int(n), c_int(k), c_int(_sm_count(a.device)), ptr(_status_word(a.device)), stream())
+            None if pads else ptr(plan.counts), None if pads else ptr(plan.offsets), c_int(int(glu)), c_int(rows // PAD),
+            c_int(n), c_int(k), c_int(_sm_count(a.device)), ptr(_status_word(a.device)), stream())
         if rc != _NOT_SUPPORTED:
             check(rc, "moe_grouped_gemm")
             return c
+    if glu:
+        from .elementwise import swiglu_fwd
+        act = swiglu_fwd(grouped_gemm(a, plan, b2d, True, ex, ey, 2 * n, pads=pads))
+        return act if out is None else out.copy_(act)
     c = torch.zeros(rows, n, dtype=a.dtype, device=a.device) if out is None else out.zero_()
     counts, offsets = plan.counts.tolist(), plan.offsets.tolist()
     for e, cnt in enumerate(counts):
@@ -233,15 +242,15 @@ def grouped_gemm(a: torch.Tensor, plan: MoePlan, b2d: torch.Tensor, b_mn_major: 
     return c
 
 
-def grouped_gemm_nt(a: torch.Tensor, plan: MoePlan, w: torch.Tensor) -> torch.Tensor:
-    """``c[r] = a[r] @ w[e].T`` for the rows of expert e, ``w [E, N, K]`` contiguous.  bf16 shapes that fit the
+def grouped_gemm_nt(a: torch.Tensor, plan: MoePlan, w: torch.Tensor, pads: bool = True) -> torch.Tensor:
+    """``c[r] = a[r] @ w[e].T`` for the rows of expert e, ``w [E, N, K]`` contiguous (``pads`` as in :func:`grouped_gemm`).  bf16 shapes that fit the
     tcgen05 kernel run there; fp32 (true 32-bit products) and other bf16 shapes on the CUDA cores
     (``csrc/grouped_gemm_simt.cu``).  Nothing is read back to the host."""
     e, n, k = w.shape
     if not _lib.use_kernels(a, w):
         return grouped_gemm(a, plan, w.reshape(e * n, k), False, 0, n, n)
     if a.dtype == torch.bfloat16 and k % 64 == 0 and n % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
-        return grouped_gemm(a, plan, w.view(e * n, k), False, 0, n, n)
+        return grouped_gemm(a, plan, w.view(e * n, k), False, 0, n, n, pads=pads)
     assert a.is_contiguous() and w.is_contiguous() and a.shape == (plan.max_rows, k) and a.dtype == w.dtype
     c = guard.empty(plan.max_rows, n, dtype=a.dtype, device=a.device)
     check(_lib.load().msrl_grouped_gemm_simt(ptr(a), ptr(w), ptr(c), c_int(plan.max_rows), c_int(n), c_int(k),

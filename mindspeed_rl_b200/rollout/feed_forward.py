@@ -59,9 +59,9 @@ class GroupedExperts:
     def run(self, h: torch.Tensor, plan: K.MoePlan, input_w: Optional[torch.Tensor] = None
             ) -> Tuple[torch.Tensor, K.MoePlan, Optional[torch.Tensor]]:
         s = self.spec
-        gu = K.grouped_gemm_nt(K.moe_permute(h, plan, input_w), plan, self.w1)
+        gu = K.grouped_gemm_nt(K.moe_permute(h, plan, input_w, zero_pads=False), plan, self.w1, pads=False)
         act = ops.glu_fwd(gu, s.expert.act, s.expert.limit, s.expert.alpha, plan=plan)
-        y = K.grouped_gemm_nt(act, plan, self.w2)
+        y = K.grouped_gemm_nt(act, plan, self.w2, pads=False)
         return y, plan, self.shared(h) if self.shared is not None else None
 
     def finish_(self, resid, h, done, norm, delta: Optional[torch.Tensor] = None) -> torch.Tensor:

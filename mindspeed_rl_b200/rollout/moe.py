@@ -64,8 +64,9 @@ class MoEWeights:
             from ..ops import moe as K
             h, f = x.shape[1], self.w2.shape[1]
             plan = K.moe_plan(phys, n_phys)
-            gu = K.grouped_gemm(K.moe_permute(x, plan), plan, self.w1.reshape(h, n_phys * 2 * f), True, 2 * f, 0, 2 * f)
-            y = K.grouped_gemm(ops.swiglu_fwd(gu), plan, self.w2.reshape(n_phys * f, h), True, 0, f, h)
+            act = K.grouped_gemm(K.moe_permute(x, plan, zero_pads=False), plan, self.w1.reshape(h, n_phys * 2 * f), True, 2 * f, 0, f,
+                                 pads=False, glu=True)
+            y = K.grouped_gemm(act, plan, self.w2.reshape(n_phys * f, h), True, 0, f, h, pads=False)
             out = K.moe_combine(y, plan, top_p)
             return self._add_shared(out, x, comm, fork)
         disp = self.p2p(x) if (self.p2p is not None and self.ep_size > 1) else None

@@ -208,3 +208,32 @@ def test_rollout_moe_with_shared_experts_on_side_stream():
     torch.cuda.synchronize()
     assert torch.equal(out, layer.forward(static_x))
     G.check_status("cuda", "rollout moe")
+
+
+@pytest.mark.parametrize("t,k,e,h,f", [(1, 1, 3, 64, 8), (48, 8, 128, 256, 192), (31, 2, 4, 128, 72), (700, 3, 5, 192, 320), (1500, 1, 2, 64, 136)])
+def test_grouped_gemm_without_pads(t, k, e, h, f):
+    """Pad rows left out (nan in their place reaches no row of a token) and SwiGLU in the epilogue: the bits of the plain kernels,
+    with segments of 1 to several hundred rows and widths that end inside a tile."""
+    from mindspeed_rl_b200 import ops
+    torch.manual_seed(2)
+    x = torch.randn(t, h, device="cuda").bfloat16()
+    idx = torch.stack([torch.randperm(e, device="cuda")[:k] for _ in range(t)])
+    w1 = (torch.randn(h, e, 2 * f, device="cuda") * 0.1).bfloat16().view(h, e * 2 * f)
+    wt = (torch.randn(e, f, h, device="cuda") * 0.1).bfloat16()
+    plan = M.moe_plan(idx, e)
+    rows = plan.pos.long()
+    gu = M.grouped_gemm(M.moe_permute(x, plan), plan, w1, True, 2 * f, 0, 2 * f)
+    want_nt = M.grouped_gemm_nt(M.moe_permute(x, plan), plan, wt)
+    xp = M.moe_permute(x, plan, zero_pads=False)
+    pad = torch.ones(plan.max_rows, dtype=torch.bool, device="cuda")
+    pad[rows] = False
+    xp[pad] = float("nan")
+    got = {}
+    for glu in (False, True):
+        out = torch.full((plan.max_rows, f if glu else 2 * f), 5.0, device="cuda").bfloat16()
+        got[glu] = M.grouped_gemm(xp, plan, w1, True, 2 * f, 0, out.shape[1], out=out, pads=False, glu=glu)
+        assert bool((out[pad] == 5.0).all())
+    assert torch.equal(got[False][rows], gu[rows])
+    assert torch.equal(got[True][rows], ops.swiglu_fwd(gu)[rows])
+    assert torch.equal(M.grouped_gemm_nt(xp, plan, wt, pads=False)[rows], want_nt[rows])
+    G.check_status(torch.device("cuda", torch.cuda.current_device()), "grouped gemm")
