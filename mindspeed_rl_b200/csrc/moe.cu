@@ -8,7 +8,8 @@
 //   permute   x[token] (optionally scaled by the slot's weight) -> rows of the expert-grouped
 //             buffer; pad rows of every segment are zeroed.
 //   route_top the experts of the largest logits of every token, with their sigmoids or the soft-max over those chosen
-//   route_softmax_top  those of the largest soft-max score plus correction, with their scores
+//   route_softmax_top  those of the largest soft-max score plus correction, with their scores (or these over their sum)
+//   router_logits  x w^T of a few tokens, 32-bit weights and sums
 //   combine   out[token] = sum_k w[token, k] * y[row(token, k)]   (fp32 accumulation; w optional)
 //   slot_dot  dw[token, k] = <dout[token], y[row(token, k)]>      (gradient of the combine weights)
 //
@@ -206,7 +207,8 @@ __device__ __forceinline__ unsigned ordered_key(float x) {      // same order as
 // One warp per token.  Scores stay in registers, what decides (score + correction) beside them as integers.
 template <int NPL>
 __global__ void __launch_bounds__(256)
-route_softmax_top_kernel(const float* logits, const float* correction, int T, int E, int top, long long* idx, float* score) {
+route_softmax_top_kernel(const float* logits, const float* correction, int T, int E, int top, int norm, float factor,
+                         long long* idx, float* score) {
   const long long t = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
@@ -229,8 +231,9 @@ route_softmax_top_kernel(const float* logits, const float* correction, int T, in
 #pragma unroll
   for (int n = 0; n < NPL; ++n) {
     s[n] /= sum;
-    key[n] = n * 32 + lane < E ? ordered_key(s[n] + correction[n * 32 + lane]) : 0u;
+    key[n] = n * 32 + lane < E ? ordered_key(correction != nullptr ? s[n] + correction[n * 32 + lane] : s[n]) : 0u;
   }
+  float taken = 0.f;
   for (int j = 0; j < top; ++j) {
     unsigned mine = 0;
 #pragma unroll
@@ -247,8 +250,52 @@ route_softmax_top_kernel(const float* logits, const float* correction, int T, in
         key[n] = 0;
         idx[t * top + j] = first;
         score[t * top + j] = s[n];
+        taken += s[n];
       }
   }
+  if (!norm && factor == 1.f) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) taken += __shfl_xor_sync(0xffffffffu, taken, o);
+  __syncwarp();
+  for (int j = lane; j < top; j += 32) {
+    const float v = score[t * top + j];
+    score[t * top + j] = (norm ? v / (taken + 1e-20f) : v) * factor;
+  }
+}
+
+// One block per expert and sixteen tokens, its threads along the row: all a block reads is in flight after a step or two.  Bound by
+// that latency (one warp to an expert, sixteen steps one after the other, took 45 us); a library GEMM in fp32 has two blocks of
+// 64 x 64 for it: 48 tokens, 128 experts of 2048: 17.6 + 2.3 us, here 5.5.
+constexpr int ROUTER_TOKENS = 16;
+__global__ void __launch_bounds__(128)
+router_logits_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, int T, int E, int H, float* __restrict__ out) {
+  __shared__ float part[4][ROUTER_TOKENS];
+  const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t0 = blockIdx.y * ROUTER_TOKENS;
+  float acc[ROUTER_TOKENS];
+#pragma unroll
+  for (int i = 0; i < ROUTER_TOKENS; ++i) acc[i] = 0.f;
+#pragma unroll 2
+  for (int c = threadIdx.x * 4; c < H; c += 512) {
+    const float4 a = *reinterpret_cast<const float4*>(w + (long long)e * H + c);
+    uint2 raw[ROUTER_TOKENS];
+#pragma unroll
+    for (int i = 0; i < ROUTER_TOKENS; ++i) raw[i] = *reinterpret_cast<const uint2*>(x + (long long)min(t0 + i, T - 1) * H + c);
+#pragma unroll
+    for (int i = 0; i < ROUTER_TOKENS; ++i) {
+      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[i].x));
+      const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[i].y));
+      acc[i] = fmaf(a.w, hi.y, fmaf(a.z, hi.x, fmaf(a.y, lo.y, fmaf(a.x, lo.x, acc[i]))));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < ROUTER_TOKENS; ++i) {
+    const float s = warp_sum(acc[i]);
+    if (lane == 0) part[warp][i] = s;
+  }
+  __syncthreads();
+  const int i = threadIdx.x;
+  if (i < ROUTER_TOKENS && t0 + i < T)
+    out[(long long)(t0 + i) * E + e] = (part[0][i] + part[1][i]) + (part[2][i] + part[3][i]);
 }
 
 __global__ void __launch_bounds__(128)
@@ -353,18 +400,29 @@ MSRL_API int msrl_route_top(const float* logits, int T, int E, int top, long lon
                 : go(route_top_kernel<2, false>, route_top_kernel<8, false>, route_top_kernel<32, false>);
 }
 
-// logits [T, E], correction [E] -> idx, score [T, top]; at most 1024 router outputs
-MSRL_API int msrl_route_softmax_top(const float* logits, const float* correction, int T, int E, int top, long long* idx,
-                                    float* score, cudaStream_t st) {
+// logits [T, E], correction [E] (or null) -> idx, score [T, top], with `norm` over their sum, times `factor`; at most 1024 router
+// outputs
+MSRL_API int msrl_route_softmax_top(const float* logits, const float* correction, int T, int E, int top, int norm, float factor,
+                                    long long* idx, float* score, cudaStream_t st) {
   if (T == 0) return 0;
   if (E < 1 || E > 1024 || top < 1 || top > E) return (int)cudaErrorInvalidValue;
-  const unsigned grid = (unsigned)((T + 7) / 8);
-  if (E <= 32) route_softmax_top_kernel<1><<<grid, 256, 0, st>>>(logits, correction, T, E, top, idx, score);
-  else if (E <= 64) route_softmax_top_kernel<2><<<grid, 256, 0, st>>>(logits, correction, T, E, top, idx, score);
-  else if (E <= 96) route_softmax_top_kernel<3><<<grid, 256, 0, st>>>(logits, correction, T, E, top, idx, score);
-  else if (E <= 160) route_softmax_top_kernel<5><<<grid, 256, 0, st>>>(logits, correction, T, E, top, idx, score);
-  else if (E <= 288) route_softmax_top_kernel<9><<<grid, 256, 0, st>>>(logits, correction, T, E, top, idx, score);
-  else route_softmax_top_kernel<32><<<grid, 256, 0, st>>>(logits, correction, T, E, top, idx, score);
+  auto* kernel = E <= 32    ? route_softmax_top_kernel<1>
+                 : E <= 64  ? route_softmax_top_kernel<2>
+                 : E <= 96  ? route_softmax_top_kernel<3>
+                 : E <= 160 ? route_softmax_top_kernel<5>
+                 : E <= 288 ? route_softmax_top_kernel<9>
+                            : route_softmax_top_kernel<32>;
+  kernel<<<(unsigned)((T + 7) / 8), 256, 0, st>>>(logits, correction, T, E, top, norm, factor, idx, score);
+  return (int)cudaGetLastError();
+}
+
+// x [T, H] bf16, w [E, H] fp32 -> out [T, E] fp32; contiguous, H a multiple of 4, x aligned to 8 bytes, w to 16
+MSRL_API int msrl_router_logits(const void* x, const float* w, int T, int E, int H, float* out, cudaStream_t st) {
+  if (T == 0 || E == 0) return 0;
+  const int tiles = (T + ROUTER_TOKENS - 1) / ROUTER_TOKENS;
+  if (H % 4 != 0 || tiles > 65535 || (reinterpret_cast<uintptr_t>(x) & 7) != 0 || (reinterpret_cast<uintptr_t>(w) & 15) != 0)
+    return (int)cudaErrorInvalidValue;
+  router_logits_kernel<<<dim3((unsigned)E, (unsigned)tiles), 128, 0, st>>>((const __nv_bfloat16*)x, w, T, E, H, out);
   return (int)cudaGetLastError();
 }
 

@@ -19,7 +19,7 @@ import torch
 from . import guard
 
 from . import _lib
-from ._lib import c_int, c_ll, check, ptr, stream
+from ._lib import c_float, c_int, c_ll, check, ptr, stream
 
 PAD = 128
 _NOT_SUPPORTED = 801
@@ -92,21 +92,40 @@ def route_top(logits: torch.Tensor, top: int, chosen_softmax: bool = False) -> T
     return idx[:, :top].contiguous(), torch.softmax(z, dim=-1) if chosen_softmax else torch.sigmoid(z)
 
 
-def route_softmax_top(logits: torch.Tensor, correction: torch.Tensor, top: int) -> Tuple[torch.Tensor, torch.Tensor]:
+def route_softmax_top(logits: torch.Tensor, correction: Optional[torch.Tensor], top: int, norm: bool = False,
+                      factor: float = 1.0) -> Tuple[torch.Tensor, torch.Tensor]:
     """Router logits ``[T, E]`` fp32 -> ``(ids [T, top] int64, scores [T, top] fp32)``: the ``top`` largest of
-    ``softmax(logits) + correction`` in descending order (equal ones: the lower id first) with their soft-max scores,
-    which the correction does not enter and which are not renormalised."""
+    ``softmax(logits) (+ correction)`` in descending order (equal ones: the lower id first) with their soft-max scores,
+    which the correction does not enter, divided by their sum with ``norm``, times ``factor``."""
     t, e = logits.shape
-    if _lib.use_kernels(logits, correction):
+    if _lib.use_kernels(logits):
         logits = logits.contiguous()
         idx = guard.empty(t, top, dtype=torch.int64, device=logits.device)
         score = guard.empty(t, top, dtype=torch.float32, device=logits.device)
-        check(_lib.load().msrl_route_softmax_top(ptr(logits), ptr(correction), c_int(t), c_int(e), c_int(top), ptr(idx),
-                                                 ptr(score), stream()), "route_softmax_top")
+        check(_lib.load().msrl_route_softmax_top(ptr(logits), ptr(correction), c_int(t), c_int(e), c_int(top), c_int(int(norm)),
+                                                 c_float(factor), ptr(idx), ptr(score), stream()), "route_softmax_top")
         return idx, score
     s = torch.softmax(logits, dim=-1)
-    idx = torch.sort(s + correction, dim=-1, descending=True, stable=True).indices[:, :top].contiguous()
-    return idx, s.gather(1, idx)
+    pick = s if correction is None else s + correction
+    idx = torch.sort(pick, dim=-1, descending=True, stable=True).indices[:, :top].contiguous()
+    s = s.gather(1, idx)
+    return idx, (s / (s.sum(-1, keepdim=True) + 1e-20) if norm else s) * factor
+
+
+ROUTER_ROWS = 256       # tokens up to which router_logits has a kernel of its own
+
+
+def router_logits(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """``x [T, H] @ w [E, H].T`` with 32-bit products and sums (``[T, E]`` fp32), whatever the operands' types."""
+    t, h = x.shape
+    if (x.is_cuda and 0 < t <= ROUTER_ROWS and x.dtype == torch.bfloat16 and w.dtype == torch.float32 and h % 4 == 0
+            and x.is_contiguous() and w.is_contiguous() and x.data_ptr() % 8 == 0 and w.data_ptr() % 16 == 0
+            and _lib.use_kernels(x, w)):
+        out = guard.empty(t, w.shape[0], dtype=torch.float32, device=x.device)
+        check(_lib.load().msrl_router_logits(ptr(x), ptr(w), c_int(t), c_int(w.shape[0]), c_int(h), ptr(out), stream()),
+              "router_logits")
+        return out
+    return torch.matmul(x.float(), w.float().t())
 
 
 def moe_permute(x: torch.Tensor, plan: MoePlan, w: Optional[torch.Tensor] = None, zero_pads: bool = True) -> torch.Tensor:

@@ -48,13 +48,25 @@ class MoEWeights:
         slot = torch.arange(top_idx.numel(), device=top_idx.device).view_as(top_idx) % n_rep[top_idx]
         return table[top_idx, slot]
 
+    def _route(self, x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+        from ..ops import moe as K
+
+        cfg = self.cfg
+        logits = K.router_logits(x, self.router_w)
+        if (cfg.moe_router_score_function == "sigmoid" or (cfg.moe_router_num_groups and cfg.moe_router_group_topk)
+                or not logits.is_cuda or logits.shape[1] > 1024):
+            return route(logits, cfg, self.expert_bias)[:2]
+        bias = None if self.expert_bias is None else self.expert_bias.float().contiguous()
+        idx, score = K.route_softmax_top(logits, bias, cfg.moe_router_topk, bool(cfg.norm_topk_prob),
+                                         float(cfg.moe_router_topk_scaling_factor or 1.0))
+        return score, idx
+
     @torch.no_grad()
     def forward(self, x: torch.Tensor, comm=None) -> torch.Tensor:
         cfg = self.cfg
         t, k = x.shape[0], cfg.moe_router_topk
         fork = self._fork_shared(x)
-        logits = torch.matmul(x.float(), self.router_w.float().t())
-        top_p, top_idx, _ = route(logits, cfg, self.expert_bias)
+        top_p, top_idx = self._route(x)
         if self.collect_counts:
             self.counts += torch.bincount(top_idx.reshape(-1).cpu(), minlength=cfg.num_experts)
         phys = self._physical(top_idx)

@@ -237,3 +237,23 @@ def test_grouped_gemm_without_pads(t, k, e, h, f):
     assert torch.equal(got[True][rows], ops.swiglu_fwd(gu)[rows])
     assert torch.equal(M.grouped_gemm_nt(xp, plan, wt, pads=False)[rows], want_nt[rows])
     G.check_status(torch.device("cuda", torch.cuda.current_device()), "grouped gemm")
+
+
+@pytest.mark.parametrize("t,e,h,k", [(1, 128, 2048, 8), (15, 60, 132, 4), (16, 1, 64, 1), (17, 130, 256, 6), (256, 512, 1024, 9)])
+@pytest.mark.parametrize("norm,factor,biased", [(True, 1.0, False), (False, 2.5, True), (True, 0.5, True)])
+def test_router_of_few_tokens(t, e, h, k, norm, factor, biased):
+    """Router logits with 32-bit sums and the choice with renormalised, scaled scores, against 64 bits and plain torch."""
+    torch.manual_seed(3)
+    x = torch.randn(t, h, device="cuda").bfloat16()
+    w = torch.randn(e, h, device="cuda") * h ** -0.5
+    bias = 0.01 * torch.randn(e, device="cuda") if biased else None
+    logits = M.router_logits(x, w)
+    exact = x.double() @ w.double().t()
+    # sums of h products in 32 bits: a chain of h / 32 and a tree, errors of a few 2^-24 of the terms' magnitudes
+    assert (logits - exact).abs().max().item() <= 2 ** -20 * (x.double().abs() @ w.double().abs().t()).max().item()
+    idx, score = M.route_softmax_top(logits, bias, k, norm, factor)
+    s = torch.softmax(logits, -1)
+    want = (s if bias is None else s + bias).topk(k, -1).indices
+    assert torch.equal(torch.sort(idx, -1).values, torch.sort(want, -1).values)
+    p = s.gather(1, idx)
+    torch.testing.assert_close(score, (p / p.sum(-1, keepdim=True) if norm else p) * factor, rtol=1e-5, atol=1e-7)
