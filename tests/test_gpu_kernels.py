@@ -97,6 +97,32 @@ def test_headnorm_and_rope(interleaved):
     close(dw, dwr, 0.3, 3e-2, "headnorm dw")
 
 
+@pytest.mark.parametrize("hd", [64, 72, 128, 136, 256])
+@pytest.mark.parametrize("t,nh,nkv", [(1, 1, 1), (7, 3, 1), (1001, 8, 2), (1500, 12, 4)])
+def test_headnorm_and_rope_sizes(hd, t, nh, nkv):
+    """Head sizes on both sides of 8, 16 and 32 lanes to a head (and of 16 entries for the rotation), head counts that end inside a
+    block, one and several heads a thread."""
+    torch.manual_seed(2)
+    lay = QKVLayout(nh, nkv, hd, True)
+    qkv, dq = (torch.randn(t, lay.width, device=DEV).bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(hd, device=DEV)).bfloat16()
+    pos = torch.randint(0, 300, (t,), device=DEV, dtype=torch.int32)
+    a, b = qkv.clone(), qkv.cpu()
+    da, db = dq.clone(), dq.cpu()
+    for which in ("q", "k"):
+        r1, r2 = ops.headnorm_fwd_(a, lay, which, w, 1e-6), ops.headnorm_fwd_(b, lay, which, w.cpu(), 1e-6)
+        close(r1, r2, 1e-3, 1e-2, "rstd " + which)
+        dw, dwr = torch.zeros(hd, device=DEV), torch.zeros(hd)
+        ops.headnorm_bwd_(da, qkv, lay, which, w, r1, dw)
+        ops.headnorm_bwd_(db, qkv.cpu(), lay, which, w.cpu(), r1.cpu(), dwr)
+        close(dw, dwr, 2e-3 * math.sqrt(t * nh) + 1e-2, 1e-2, "dw " + which)
+    close(a, b, 3e-2, 2e-2, "headnorm")
+    close(da, db, 3e-2, 3e-2, "headnorm dx")
+    ops.rope_(a, lay, pos, ops.rope_table(300, hd, 1e4, DEV))
+    ops.rope_(b, lay, pos.cpu(), ops.rope_table(300, hd, 1e4, "cpu"))
+    close(a, b, 4e-2, 2e-2, "rope")
+
+
 def test_swiglu_and_colsum():
     torch.manual_seed(2)
     x = torch.randn(77, 2 * 1536, device=DEV, dtype=torch.bfloat16)
