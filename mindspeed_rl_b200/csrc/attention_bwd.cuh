@@ -193,7 +193,7 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         l[i] = q < qlen ? -__ldg(p.lse + at) * LOG2E : -INFINITY;      // P is exactly 0
         d[i] = q < qlen ? -__ldg(p.delta + at) : 0.f;
       }
-      if (use > 0 && !mbar_wait(&q_empty[st], (use - 1) & 1, p.error, ERR_EMPTY)) break;
+      if (use > 0 && !mbar_wait_warp(&q_empty[st], (use - 1) & 1, p.error, ERR_EMPTY)) break;   // all lanes or none
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         stat[st][0][i * 32 + lane] = l[i];
