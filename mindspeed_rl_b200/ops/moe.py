@@ -98,7 +98,7 @@ def route_softmax_top(logits: torch.Tensor, correction: Optional[torch.Tensor], 
     ``softmax(logits) (+ correction)`` in descending order (equal ones: the lower id first) with their soft-max scores,
     which the correction does not enter, divided by their sum with ``norm``, times ``factor``."""
     t, e = logits.shape
-    if _lib.use_kernels(logits):
+    if _lib.use_kernels(logits, correction):
         logits = logits.contiguous()
         idx = guard.empty(t, top, dtype=torch.int64, device=logits.device)
         score = guard.empty(t, top, dtype=torch.float32, device=logits.device)

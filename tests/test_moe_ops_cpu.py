@@ -62,3 +62,14 @@ def test_permute_grouped_gemm_combine_matches_dense_loop():
     dout = torch.randn(t, h)
     dw = M.moe_slot_dot(dout, y, plan)
     torch.testing.assert_close(dw[5, 1], (dout[5] * y[int(plan.pos[5 * k + 1])]).sum(), rtol=1e-4, atol=1e-4)
+
+
+def test_route_softmax_top_asks_for_the_correction_on_the_device_too(monkeypatch):
+    """The kernel reads the correction by its address: where it lies on the host the kernel must not be taken."""
+    asked = []
+    monkeypatch.setattr(M._lib, "use_kernels", lambda *t: asked.append(t) or False)
+    logits, correction = torch.randn(5, 8), torch.randn(8)
+    M.route_softmax_top(logits, correction, 2)
+    assert any(x is correction for x in asked[0])
+    idx, score = M.route_softmax_top(logits, None, 2)
+    assert torch.equal(idx, logits.topk(2).indices) and score.shape == (5, 2)
