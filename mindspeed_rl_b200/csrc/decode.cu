@@ -932,11 +932,18 @@ MSRL_API int msrl_kv_cache_gather(const void* k_cache, const void* v_cache, cons
 // piece.  Kernel alone, heads of 128, 4096 keys at most: 48 sequences of 701 to 3700 keys, 4 KV heads, 1 / 2 / 3 / 4 / 8 / 16 pieces:
 // 66 / 53 / 48 / 47 / 49 / 57 us; 256 of 1 to 1024: 60 / 68 / 68 / 74; 8 of 500 to 2000: 28 / 16 / 12 / 10 / 9 / 10; 1 of 2924: 40
 // alone, 6 in 16.  (Pieces that filled whole waves, the rule before: 8, 2, 8 and 16.)
+// `max_ctx` is a bound: a captured step passes the longest sequence that the engine allows, whatever its sequences hold.  Where the
+// blocks fill the machine without pieces it counts up to 8192 keys only.  256 sequences, 4 KV heads of 128, bound of 32768, 2 / 4
+// pieces (whole waves: 2): 64 to 1024 keys 72 / 84 us (74), 700 to 3700 201 / 205 (220), 1000 to 16000 724 / 705 (779); 128 sequences,
+// 3 / 6 pieces (4): 44 / 52 (50), 110 / 117 (120), 337 / 323 (353); 256 sequences, 8 heads of 64, 1 / 3 pieces (1): 62 / 79 (64),
+// 213 / 218 (232), 814 / 778 (880).  With blocks to spare it counts up to 32768, the longest bound that was measured.
 MSRL_API int msrl_paged_decode_nsplit(int B, int nkv, int max_ctx) {
+  const double slots = 2.0 * sm_count(), blocks = B * (double)nkv;
+  const int bound = blocks >= slots ? 8192 : 32768, longest = max_ctx < bound ? max_ctx : bound;
   int best = 1;
   double best_cost = 1e30;
   for (int ns = 1; ns <= 32 && (ns == 1 || max_ctx >= 256 * ns); ++ns) {
-    const double cost = 2.5 * ns * B * (double)nkv / (2.0 * sm_count()) + 0.0042 * max_ctx / ns + (ns > 1 ? 3.0 : 0.0);
+    const double cost = 2.5 * ns * blocks / slots + 0.0042 * longest / ns + (ns > 1 ? 3.0 : 0.0);
     if (cost < best_cost) best = ns, best_cost = cost;
   }
   return best;

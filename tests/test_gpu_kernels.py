@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from mindspeed_rl_b200 import ops
-from mindspeed_rl_b200.ops import QKVLayout
+from mindspeed_rl_b200.ops import QKVLayout, _lib
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -222,6 +222,17 @@ def test_paged_decode_pieces(nh, nkv, hd, bs, lens):
     out = ops.paged_decode_attention(qkv, lay, kc, vc, bt, ctx, 4096)
     ref = ops.paged_decode_attention(qkv.cpu(), lay, kc.cpu(), vc.cpu(), bt.cpu(), ctx.cpu(), 4096)
     close(out, ref, 2e-2, 2e-2, "out")
+
+
+def test_paged_decode_pieces_under_a_long_bound():
+    """A bound on the context far above what the sequences hold (the engine's limit in a captured step): a machine that is full
+    without pieces is not cut further for it, one with blocks to spare still is."""
+    pieces = _lib.load().msrl_paged_decode_nsplit
+    for b, nkv in ((256, 4), (128, 8), (128, 4), (96, 4), (256, 8)):
+        assert pieces(b, nkv, 32768) == pieces(b, nkv, 131072) == pieces(b, nkv, 8192) <= 3
+        assert pieces(b, nkv, 1024) <= pieces(b, nkv, 4096) <= pieces(b, nkv, 8192)
+    assert pieces(1, 4, 32768) == pieces(1, 4, 1 << 20) == 32
+    assert [pieces(b, 4, 131072) == pieces(b, 4, 32768) for b in (4, 8, 32, 64)] == [True] * 4
 
 
 @pytest.mark.parametrize("nh,nkv,hd,bs,n_samples,prompt", [(28, 4, 128, 16, 8, 200), (8, 2, 64, 16, 5, 70),
