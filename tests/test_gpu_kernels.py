@@ -123,6 +123,21 @@ def test_headnorm_and_rope_sizes(hd, t, nh, nkv):
     close(a, b, 4e-2, 2e-2, "rope")
 
 
+@pytest.mark.parametrize("t", [1, 3, 257])
+@pytest.mark.parametrize("nh,nkv,hd", [(32, 4, 128), (32, 8, 128), (5, 1, 256), (3, 3, 24)])
+def test_rope_head_counts(nh, nkv, hd, t):
+    """Tokens whose vectors end inside a block of 256 threads, with separate and with interleaved heads, forward and back."""
+    torch.manual_seed(3)
+    for interleaved in (True, False):
+        lay = QKVLayout(nh, nkv, hd, interleaved)
+        a = torch.randn(t, lay.width, device=DEV).bfloat16()
+        b, pos = a.cpu(), torch.randint(0, 90, (t,), device=DEV, dtype=torch.int32)
+        for inverse in (False, True):
+            ops.rope_(a, lay, pos, ops.rope_table(90, hd, 1e4, DEV), inverse=inverse)
+            ops.rope_(b, lay, pos.cpu(), ops.rope_table(90, hd, 1e4, "cpu"), inverse=inverse)
+            close(a, b, 4e-2, 2e-2, "rope")
+
+
 def test_swiglu_and_colsum():
     torch.manual_seed(2)
     x = torch.randn(77, 2 * 1536, device=DEV, dtype=torch.bfloat16)
