@@ -27,6 +27,7 @@
 #include <cudaTypedefs.h>
 #include <stdlib.h>
 
+#include "row_stat.cuh"
 #include "tcgen05_utils.cuh"
 
 namespace msrl {
@@ -52,11 +53,6 @@ constexpr int COMM_THREADS = 128;     // four extra warps move data over NVLink 
 constexpr int AG_PIECES = 16;         // a 128-row unit is gathered as 16 pieces of 8 rows
 constexpr int RS_CHUNKS = 16;         // a 128-row unit is reduced as 16 column chunks
 
-// of one row over the 256 columns of a tile: largest logit, sum of exp, the label's logit (0 elsewhere), sum of exp * logit
-struct RowStat4 {
-  float m, s, zy, spz;
-};
-
 struct Params {
   int M, N, K;
   void* C;
@@ -78,7 +74,7 @@ struct Params {
   const long long* labels;     // [M] global vocabulary ids
   int vocab_offset;            // id of column 0
   float inv_temp;
-  RowStat4* stats;             // [column tiles, M]
+  RowStat* stats;              // [column tiles, M]
   // communication-fused variants (tensor-parallel linears under sequence parallelism)
   int rank, world;
   int m_local;                 // rows owned by one rank (multiple of 256); M = world * m_local
@@ -506,43 +502,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           flush(reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, n0 + c * 64);
         }
       } else if constexpr (OUT == OUT_STATS) {
-        float mx = -INFINITY, s = 0.f, spz = 0.f, zy = 0.f;
         const long long label = (row < p.M) ? p.labels[row] - p.vocab_offset : -1;
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          float v[32];
-          tmem_ld32(t_row + c * 32, v);
-          const int col = n0 + c * 32;
-          float cm = -INFINITY;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            // logits take the bf16 rounding the un-fused path would apply before the soft-max
-            v[j] = (col + j < p.N) ? __bfloat162float(__float2bfloat16(v[j])) * p.inv_temp : -INFINITY;
-            cm = fmaxf(cm, v[j]);
-          }
-          if (cm > mx) {
-            const float corr = __expf(mx - cm);
-            s *= corr;
-            spz *= corr;
-            mx = cm;
-          }
-          if (mx > -INFINITY) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (col + j < p.N) {
-                const float e = __expf(v[j] - mx);
-                s += e;
-                spz += e * v[j];
-              }
-            }
-          }
-          if (label >= col && label < col + 32 && label < p.N) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (label == col + j) zy = v[j];
-          }
-        }
-        if (row < p.M) p.stats[(long long)nt * p.M + row] = RowStat4{mx, s, zy, spz};
+        const RowStat r = tile_row_stat<BN>([&](int c, float (&v)[32]) { tmem_ld32(t_row + c * 32, v); }, n0, p.N, label, p.inv_temp);
+        if (row < p.M) p.stats[(long long)nt * p.M + row] = r;
       } else {
         // Accumulating epilogues (weight gradients): C += acc through the warp's shared-memory patch, so
         // that the read-modify-write of C moves whole 128-byte (fp32) / 64-byte (bf16) row segments per
@@ -876,8 +838,9 @@ MSRL_API int msrl_lmhead_stats_tiles(int N) { return (N + g2::BN - 1) / g2::BN; 
 
 // LM head fused with the log-softmax statistics: stats[column tile, M] records over 256-column tiles of z = (H W^T) * inv_temp;
 // combine them with msrl_logprob_finish(nshard = tiles * shards).  On CTA pairs, which pull half as much of W through L2 and
-// shared memory as a block alone (128 x 256 tiles before): 16384 tokens, 152064 x 3584: 16038 -> 12932 us
-// (1381 TFLOP/s), 4096 tokens 2789 -> 2683, 1500 tokens 1075 -> 1069, 300 tokens (512 rows of tiles, 384 before) 309 -> 359.
+// shared memory as a block alone (128 x 256 tiles before): 16384 tokens, 152064 x 3584: 16038 -> 12932 us (1381 TFLOP/s).  Where
+// the last 256 rows are at most half full, or the inner size is small, the caller takes the form with row tiles of 128
+// (gemm_tcgen05.cu).
 MSRL_API int msrl_lmhead_stats(const void* H, long long ldh, const void* W, long long ldw, const long long* labels,
                                int vocab_offset, float inv_temp, void* stats, int M, int N, int K, int* error,
                                cudaStream_t st) {
@@ -888,7 +851,7 @@ MSRL_API int msrl_lmhead_stats(const void* H, long long ldh, const void* W, long
   p.labels = labels;
   p.vocab_offset = vocab_offset;
   p.inv_temp = inv_temp;
-  p.stats = (g2::RowStat4*)stats;
+  p.stats = (RowStat*)stats;
   p.error = error;
   return g2::launch<false, false, g2::OUT_STATS>(H, ldh, W, ldw, p, st);
 }

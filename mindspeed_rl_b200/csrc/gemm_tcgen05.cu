@@ -4,8 +4,12 @@
 //   4-stage shared-memory ring guarded by full/empty mbarriers;
 // * one elected thread issues tcgen05.mma (cta_group::1, 128x256x16) on UMMA shared-memory
 //   descriptors; tcgen05.commit releases ring slots and finally signals the epilogue;
-// * four epilogue warps read the 128x256 fp32 accumulator out of TMEM with tcgen05.ld, convert to bf16 and
-//   store C.
+// * four epilogue warps read the 128x256 fp32 accumulator out of TMEM with tcgen05.ld and apply
+//   a fused epilogue:
+//     - STORE: convert to bf16 and store C;
+//     - LOGPROB_STATS: LM-head fused with the log-softmax statistics -- every row's running
+//       (max, sum-exp, target logit, sum e^z z) over this tile's 256 vocabulary columns is
+//       written as one 16-byte record; the logits themselves never reach global memory.
 //
 // Every wait on an mbarrier is bounded (wall-clock limit); on expiry the kernel records an error
 // code, skips the remaining work, still frees its TMEM allocation and returns, so the host sees
@@ -31,7 +35,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
-#include "common.cuh"
+#include "row_stat.cuh"
 
 namespace msrl {
 
@@ -161,10 +165,18 @@ constexpr uint32_t make_idesc_bf16(int m, int n) {
          | ((uint32_t)(m >> 4) << 24);  // M / 16
 }
 
+enum Epilogue { EPI_STORE = 0, EPI_LOGPROB_STATS = 1 };
+
 struct GemmParams {
   int M, N, K;
+  // EPI_STORE
   __nv_bfloat16* C;
   long long ldc;
+  // EPI_LOGPROB_STATS
+  const long long* labels;  // [M] global vocabulary ids
+  int vocab_offset;         // first vocabulary id of column 0
+  float inv_temp;
+  RowStat* stats;           // [num_n_tiles, M]
   int* error;               // device status word (0 = ok)
   // communication-fused variants
   int rank, world;
@@ -236,7 +248,7 @@ __device__ __forceinline__ void tile_coords(int tile, int m_tiles, int n_tiles, 
   }
 }
 
-template <int COMM>
+template <int EPI, int COMM>
 __global__ void __launch_bounds__(COMM == COMM_NONE ? 192 : 192 + G_COMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_a_local, const __grid_constant__ GemmParams p) {
@@ -361,7 +373,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       tcgen05_fence_after();
       const int row = m0 + warp * 32 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(warp * 32) << 16) + buf * G_BN;
-      {
+      if (EPI == EPI_STORE) {
         __nv_bfloat16* cbase = p.C;
         long long ldc = p.ldc, crow = row;
         if (COMM == COMM_RS) {
@@ -417,6 +429,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           __syncwarp();
           if (lane == 0) red_release_sys_add(p.peer_flag[mt / mt_local] + (mt % mt_local), 1u);
         }
+      } else {
+        const long long label = (row < p.M) ? p.labels[row] - p.vocab_offset : -1;
+        const RowStat r = tile_row_stat<G_BN>([&](int c, float (&v)[32]) { tmem_ld32(t_row + c * 32, v); }, n0, p.N, label, p.inv_temp);
+        if (row < p.M) p.stats[(long long)nt * p.M + row] = r;
       }
       // hand the accumulator back to the MMA warp
       tcgen05_fence_before();
@@ -556,7 +572,7 @@ static bool make_map(CUtensorMap* map, const void* base, long long rows, long lo
   return r == CUDA_SUCCESS;
 }
 
-template <int COMM = COMM_NONE>
+template <int EPI, int COMM = COMM_NONE>
 static int launch_gemm(const void* A, long long lda, const void* B, long long ldb, const GemmParams& p,
                        cudaStream_t st, const void* A_local = nullptr, long long lda_local = 0) {
   CUtensorMap ma, mb, ml;
@@ -566,7 +582,7 @@ static int launch_gemm(const void* A, long long lda, const void* B, long long ld
   if (A_local != nullptr && !make_map(&ml, A_local, p.m_local, p.K, lda_local, G_BM))
     return (int)cudaErrorInvalidValue;
   const size_t smem = (size_t)G_STAGES * G_STAGE_BYTES + G_EPI_BYTES + 1024;
-  cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<COMM>,
+  cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<EPI, COMM>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const int tiles = ((p.M + G_BM - 1) / G_BM) * ((p.N + G_BN - 1) / G_BN);
@@ -574,7 +590,7 @@ static int launch_gemm(const void* A, long long lda, const void* B, long long ld
   // work of the whole grid, and every CTA must be resident for the counters to advance.
   const int grid = (COMM != COMM_NONE || tiles >= sm_count()) ? sm_count() : tiles;
   const int threads = COMM == COMM_NONE ? 192 : 192 + G_COMM_THREADS;
-  gemm_tcgen05_kernel<COMM><<<grid, threads, smem, st>>>(ma, mb, ml, p);
+  gemm_tcgen05_kernel<EPI, COMM><<<grid, threads, smem, st>>>(ma, mb, ml, p);
   return (int)cudaGetLastError();
 }
 
@@ -593,7 +609,24 @@ MSRL_API int msrl_gemm_bf16_tn(const void* A, long long lda, const void* B, long
   p.C = (__nv_bfloat16*)C;
   p.ldc = ldc;
   p.error = error;
-  return launch_gemm(A, lda, B, ldb, p, st);
+  return launch_gemm<EPI_STORE>(A, lda, B, ldb, p, st);
+}
+
+// msrl_lmhead_stats (gemm2cta_tcgen05.cu) with row tiles of 128: the same records.  152064 columns, K = 3584: 300 rows 335 us where
+// pairs of CTAs, which compute 512 rows for them, take 361.
+MSRL_API int msrl_lmhead_stats_rows128(const void* H, long long ldh, const void* W, long long ldw, const long long* labels,
+                                       int vocab_offset, float inv_temp, void* stats, int M, int N, int K, int* error,
+                                       cudaStream_t st) {
+  if (M == 0 || N == 0) return 0;
+  if (K % 8 != 0) return (int)cudaErrorInvalidValue;
+  GemmParams p{};
+  p.M = M; p.N = N; p.K = K;
+  p.labels = labels;
+  p.vocab_offset = vocab_offset;
+  p.inv_temp = inv_temp;
+  p.stats = (RowStat*)stats;
+  p.error = error;
+  return launch_gemm<EPI_LOGPROB_STATS>(H, ldh, W, ldw, p, st);
 }
 
 // ---- communication-fused GEMMs over peer-mapped memory ------------------------------------------
@@ -620,7 +653,7 @@ MSRL_API int msrl_ag_gemm_bf16_tn(void* const* peer_a, long long ld_peer, void* 
   p.tile_ready = tile_ready;
   cudaError_t e = cudaMemsetAsync(tile_ready, 0, sizeof(unsigned int) * (size_t)(p.M / G_BM), st);
   if (e != cudaSuccess) return (int)e;
-  return launch_gemm<COMM_AG>(gathered, K, B, ldb, p, st, peer_a[rank], ld_peer);
+  return launch_gemm<EPI_STORE, COMM_AG>(gathered, K, B, ldb, p, st, peer_a[rank], ld_peer);
 }
 
 MSRL_API int msrl_gemm_rs_tiles(int N) { return (N + G_BN - 1) / G_BN; }
@@ -651,5 +684,5 @@ MSRL_API int msrl_gemm_rs_bf16_tn(const void* A, long long lda, const void* B, l
   p.rs_done = done;
   p.rs_out = (__nv_bfloat16*)out;
   p.ld_out = ld_out;
-  return launch_gemm<COMM_RS>(A, lda, B, ldb, p, st);
+  return launch_gemm<EPI_STORE, COMM_RS>(A, lda, B, ldb, p, st);
 }

@@ -6,16 +6,9 @@
 //
 // Reference semantics: vocab-parallel cross entropy and entropy with 3 all-reduces each
 // (mindspeed_rl/utils/compute.py:29-97); here the shards' 4-float records are combined once.
-#include "common.cuh"
+#include "row_stat.cuh"
 
 namespace msrl {
-
-struct RowStat {
-  float m;    // max of z over the shard
-  float s;    // sum exp(z - m)
-  float zy;   // z[label] if the label lives in this shard else 0
-  float spz;  // sum exp(z - m) * z
-};
 
 __global__ void __launch_bounds__(256)
 logprob_stats_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stride, int V,

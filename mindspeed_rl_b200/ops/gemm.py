@@ -200,6 +200,17 @@ def linear_wgrad_(grad: torch.Tensor, dy: torch.Tensor, x: torch.Tensor) -> torc
     return grad.add_(torch.matmul(dy.t(), x))
 
 
+def _lmhead_rows128(m: int, k: int) -> bool:
+    """Row tiles of 128 on single CTAs instead of 256 on pairs (one record of the same bits either way).  Pairs read the weights half
+    as often; single CTAs leave out the second half of a last tile that is at most half full, and have twice the epilogue warps to a
+    tile, which bound inner sizes below 1280 (151936 columns, K = 1024: 128 rows 94 against 80 us, 16384 rows 4966 / 4758).  Pairs /
+    single CTAs, 152064 columns, K = 3584: 1 row 248 / 213 us, 128 215 / 207, 129 215 / 246, 300 361 / 335, 640 564 / 525,
+    1152 980 / 949, 1408 1140 / 1136, 1664 1295 / 1302, 2176 1596 / 1648, 8320 6743 / 6813; K = 1536: 256 rows 136 / 142,
+    1024 411 / 394, 16384 6099 / 5942."""
+    half = (m - 1) % 256 < 128
+    return k < 1280 or (k < 1792 and (half or m > 512)) or (half and m <= 1408)
+
+
 def lmhead_stats(h: torch.Tensor, w: torch.Tensor, labels: torch.Tensor, inv_temp: float,
                  vocab_offset: int = 0) -> Tuple[torch.Tensor, int]:
     """Per-row, per-256-column-tile softmax statistics of ``(h @ w.T) * inv_temp``.
@@ -211,9 +222,9 @@ def lmhead_stats(h: torch.Tensor, w: torch.Tensor, labels: torch.Tensor, inv_tem
     L = _lib.load()
     tiles = L.msrl_lmhead_stats_tiles(c_int(n))
     stats = guard.empty(tiles, m, 4, device=h.device, dtype=torch.float32)
-    check(L.msrl_lmhead_stats(ptr(h), c_ll(h.stride(0)), ptr(w), c_ll(w.stride(0)), ptr(labels),
-                              c_int(vocab_offset), c_float(inv_temp), ptr(stats), c_int(m), c_int(n),
-                              c_int(k), ptr(_status_word(h.device)), stream()), "lmhead_stats")
+    kernel = L.msrl_lmhead_stats_rows128 if _lmhead_rows128(m, k) else L.msrl_lmhead_stats
+    check(kernel(ptr(h), c_ll(h.stride(0)), ptr(w), c_ll(w.stride(0)), ptr(labels), c_int(vocab_offset), c_float(inv_temp),
+                 ptr(stats), c_int(m), c_int(n), c_int(k), ptr(_status_word(h.device)), stream()), "lmhead_stats")
     return stats, tiles
 
 

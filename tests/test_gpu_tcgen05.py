@@ -1,10 +1,12 @@
 """tcgen05 / TMA GEMM and the fused LM-head statistics epilogue against PyTorch references."""
+import math
+
 import pytest
 import torch
 
 from mindspeed_rl_b200.ops import gemm as G
 from mindspeed_rl_b200.ops import _lib
-from mindspeed_rl_b200.ops._lib import c_int, c_ll, ptr, stream
+from mindspeed_rl_b200.ops._lib import c_float, c_int, c_ll, ptr, stream
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -120,6 +122,30 @@ def test_gemm_pair_swiglu(m, f, k):
         got, got_gu = G.linear_swiglu(x, w, keep)
         assert (got_gu is None) == (not keep)
         _assert_close(got, torch.nn.functional.silu(gate_up[:, :f].float()) * gate_up[:, f:].float(), k)
+
+
+@pytest.mark.parametrize("m", [1, 127, 128, 129, 256, 257, 300, 384, 385, 1409])
+@pytest.mark.parametrize("v,k", [(1000, 264), (2500, 1800)])
+def test_lmhead_stats_forms(m, v, k):
+    """Row tiles of 256 on CTA pairs and of 128 on single CTAs write the same records, and the rule takes the latter where the
+    last 256 rows are at most half full."""
+    torch.manual_seed(6)
+    h = torch.randn(m, k, device=DEV).bfloat16()
+    w = (torch.randn(v, k, device=DEV) * k ** -0.5).bfloat16()
+    labels = torch.randint(-5, v + 5, (m,), device=DEV)
+    got, tiles = G.lmhead_stats(h, w, labels, 0.7)
+    L = _lib.load()
+    for kernel in (L.msrl_lmhead_stats, L.msrl_lmhead_stats_rows128):
+        st = torch.full_like(got, 7.0)
+        assert kernel(ptr(h), c_ll(k), ptr(w), c_ll(k), ptr(labels), c_int(0), c_float(0.7), ptr(st), c_int(m), c_int(v), c_int(k),
+                      ptr(G._status_word(h.device)), stream()) == 0
+        assert torch.equal(st, got)
+    G.check_status(DEV)
+    z = (h.float() @ w.float().t()).bfloat16().float() * 0.7
+    pad = torch.full((m, tiles * 256 - v), -math.inf, device=DEV)
+    # a logit that lies between two bf16 values may round either way: 2^-8 of it
+    torch.testing.assert_close(got[:, :, 0].t(), torch.cat([z, pad], 1).view(m, tiles, 256).amax(-1), rtol=2 ** -7, atol=1e-3)
+    assert [G._lmhead_rows128(n, 3584) for n in (1, 128, 129, 256, 300, 640, 1664)] == [True, True, False, False, True, True, False]
 
 
 @pytest.mark.parametrize("t,v,h", [(200, 1000, 256), (513, 5000, 896)])
