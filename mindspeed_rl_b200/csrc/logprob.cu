@@ -68,46 +68,59 @@ logprob_stats_kernel(const __nv_bfloat16* __restrict__ logits, long long row_str
   }
 }
 
-// Combine `nshard` records per row ([nshard, T] layout) -> logp, entropy, lse.  A block takes 32 rows, one to a lane, and its
-// sixteen warps share the records; bound by reading them once (a thread to a row, as before, left most of the machine idle on
-// the 594 records a row of a 152064-entry vocabulary: 16384 rows 280 -> 56 us, 300 rows 104 -> 22 us).
-constexpr int FIN_WARPS = 16;
-__global__ void __launch_bounds__(FIN_WARPS * 32)
+// Combine `nshard` records per row ([nshard, T] layout) -> logp, entropy, lse.  W warps share the records of 32 rows, one row to a
+// lane; bound by reading the records once (a thread to a row, as before, left most of the machine idle on the 594 records a row of a
+// 152064-entry vocabulary: 16384 rows 211 -> 52 us, 300 rows 79 -> 15 us).  A few records a row need no sharing: see the rule below.
+template <int W, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 logprob_finish_kernel(const RowStat* __restrict__ st, int nshard, long long T, float* __restrict__ logp,
-                      float* __restrict__ entropy, float* __restrict__ lse_out) {
-  __shared__ float part[FIN_WARPS][4][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long r = (long long)blockIdx.x * 32 + lane;
+                      float* __restrict__ entropy, float* __restrict__ lse_out, bool vec) {
+  __shared__ float part[W > 1 ? WARPS : 1][4][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, mine = warp % W, first = warp - mine;
+  const long long r = ((long long)blockIdx.x * (WARPS / W) + warp / W) * 32 + lane;
   const bool on = r < T;
   float m = -INFINITY;
 #pragma unroll 4
-  for (int k = warp; k < nshard; k += FIN_WARPS)
+  for (int k = mine; k < nshard; k += W)
     if (on) m = fmaxf(m, st[(long long)k * T + r].m);
-  part[warp][0][lane] = m;
-  __syncthreads();
+  if constexpr (W > 1) {
+    part[warp][0][lane] = m;
+    __syncthreads();
 #pragma unroll
-  for (int w = 0; w < FIN_WARPS; ++w) m = fmaxf(m, part[w][0][lane]);
+    for (int w = 0; w < W; ++w) m = fmaxf(m, part[first + w][0][lane]);
+  }
   float s = 0.f, spz = 0.f, zy = 0.f;
 #pragma unroll 4
-  for (int k = warp; k < nshard; k += FIN_WARPS) {
+  for (int k = mine; k < nshard; k += W) {
     if (!on) break;
-    const float4 a = *reinterpret_cast<const float4*>(st + (long long)k * T + r);   // m, s, zy, spz
-    const float c = __expf(a.x - m);
-    s += a.y * c;
-    spz += a.w * c;
-    zy += a.z;
+    const RowStat* at = st + (long long)k * T + r;
+    RowStat a;
+    if (vec) {
+      const float4 x = *reinterpret_cast<const float4*>(at);
+      a = RowStat{x.x, x.y, x.z, x.w};
+    } else {
+      a = *at;
+    }
+    const float c = __expf(a.m - m);
+    s += a.s * c;
+    spz += a.spz * c;
+    zy += a.zy;
   }
-  part[warp][1][lane] = s;
-  part[warp][2][lane] = spz;
-  part[warp][3][lane] = zy;
-  __syncthreads();
-  if (warp != 0 || !on) return;
+  if constexpr (W > 1) {
+    part[warp][1][lane] = s;
+    part[warp][2][lane] = spz;
+    part[warp][3][lane] = zy;
+    __syncthreads();
+    if (mine == 0) {
 #pragma unroll
-  for (int w = 1; w < FIN_WARPS; ++w) {
-    s += part[w][1][lane];
-    spz += part[w][2][lane];
-    zy += part[w][3][lane];
+      for (int w = 1; w < W; ++w) {
+        s += part[first + w][1][lane];
+        spz += part[first + w][2][lane];
+        zy += part[first + w][3][lane];
+      }
+    }
   }
+  if (mine != 0 || !on) return;
   const float lse = m + __logf(s);
   logp[r] = zy - lse;
   if (entropy != nullptr) entropy[r] = lse - spz / s;
@@ -169,8 +182,17 @@ MSRL_API int msrl_logprob_stats(const void* logits, long long row_stride, long l
 MSRL_API int msrl_logprob_finish(const void* stats, int nshard, long long T, float* logp,
                                  float* entropy, float* lse, cudaStream_t st) {
   if (T == 0) return 0;
-  logprob_finish_kernel<<<(unsigned)ceil_div(T, 32), FIN_WARPS * 32, 0, st>>>((const RowStat*)stats, nshard, T, logp,
-                                                                              entropy, lse);
+  // A record a vocabulary shard: sharing costs more than it saves.  A thread to a row / 4 / 16 warps to 32 rows: 1 record, 16384 rows
+  // 1.8 / 1.9 / 2.6 us, 4 records 1.9 / 2.1 / 2.7, 8 records 2.5 / 2.3 / 2.9, 32 records 4.7 / 3.2 / 3.7 (65536 rows 9.9 / 6.0 / 9.3),
+  // 64 records 11.1 / 6.2 / 4.6.
+  const bool vec = (reinterpret_cast<uintptr_t>(stats) & 15) == 0;
+  const RowStat* in = (const RowStat*)stats;
+  if (nshard <= 4)
+    logprob_finish_kernel<1, 4><<<(unsigned)ceil_div(T, 128), 128, 0, st>>>(in, nshard, T, logp, entropy, lse, vec);
+  else if (nshard <= 32)
+    logprob_finish_kernel<4, 4><<<(unsigned)ceil_div(T, 32), 128, 0, st>>>(in, nshard, T, logp, entropy, lse, vec);
+  else
+    logprob_finish_kernel<16, 16><<<(unsigned)ceil_div(T, 32), 512, 0, st>>>(in, nshard, T, logp, entropy, lse, vec);
   MSRL_LAUNCH_CHECK();
 }
 

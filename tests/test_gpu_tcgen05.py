@@ -148,6 +148,27 @@ def test_lmhead_stats_forms(m, v, k):
     assert [G._lmhead_rows128(n, 3584) for n in (1, 128, 129, 256, 300, 640, 1664)] == [True, True, False, False, True, True, False]
 
 
+@pytest.mark.parametrize("n", [1, 4, 5, 32, 33, 600])
+@pytest.mark.parametrize("t", [1, 31, 128, 129, 700])
+def test_logprob_finish_record_counts(n, t):
+    """One, four and sixteen warps to the records of 32 rows, on both sides of their borders, from records on a 16-byte boundary and
+    beside one."""
+    torch.manual_seed(7)
+    st = torch.rand(n, t, 4, device=DEV) + 0.5
+    st[..., 0] *= 5
+    for base in (st, torch.cat([torch.zeros(1, device=DEV), st.view(-1)])[1:]):
+        logp, ent, lse = (torch.full((t,), 9.0, device=DEV) for _ in range(3))
+        assert _lib.load().msrl_logprob_finish(ptr(base), c_int(n), c_ll(t), ptr(logp), ptr(ent), ptr(lse), stream()) == 0
+        d = st.double()
+        c = torch.exp(d[..., 0] - d[..., 0].amax(0))
+        s = (d[..., 1] * c).sum(0)
+        want = d[..., 0].amax(0) + torch.log(s)
+        # fp32 sums of up to 600 terms of one sign, exponentials and logarithm on the fast units
+        torch.testing.assert_close(lse, want.float(), rtol=2e-6, atol=2e-6)
+        torch.testing.assert_close(logp, (d[..., 2].sum(0) - want).float(), rtol=1e-5, atol=1e-5)
+        torch.testing.assert_close(ent, (want - (d[..., 3] * c).sum(0) / s).float(), rtol=1e-5, atol=1e-5)
+
+
 @pytest.mark.parametrize("t,v,h", [(200, 1000, 256), (513, 5000, 896)])
 def test_lmhead_stats_fused(t, v, h):
     torch.manual_seed(1)
