@@ -112,15 +112,21 @@ def route_softmax_top(logits: torch.Tensor, correction: Optional[torch.Tensor], 
     return idx, (s / (s.sum(-1, keepdim=True) + 1e-20) if norm else s) * factor
 
 
-ROUTER_ROWS = 256       # tokens up to which router_logits has a kernel of its own
+# Tokens, and tokens times experts, up to which router_logits has a kernel of its own (blocks of sixteen tokens read the weights
+# again, the library's 64), and weights up to which it is used for one token (a product with a vector, which the library has a
+# kernel for).  Kernel / casts and library, us: 128 experts of 2048, 1 token 3 / 7, 64 5.5 / 22, 256 13.6 / 23; 256 of 7168, 1 token
+# 7.7 / 8.9, 64 20.6 / 59, 256 65 / 98; 512 of 2048, 128 tokens 24 / 38, 192 34 / 38, 256 45 / 39; 1024 of 1024, 64 tokens 16 / 22;
+# one token of 384 x 7168 8.8 / 10.0, of 512 x 7168 11.3 / 9.2, of 1024 x 7168 17.5 / 10.9.
+ROUTER_ROWS, ROUTER_LOGITS, ROUTER_VECTOR = 256, 65536, 3 << 20
 
 
 def router_logits(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """``x [T, H] @ w [E, H].T`` with 32-bit products and sums (``[T, E]`` fp32), whatever the operands' types."""
     t, h = x.shape
-    if (x.is_cuda and 0 < t <= ROUTER_ROWS and x.dtype == torch.bfloat16 and w.dtype == torch.float32 and h % 4 == 0
-            and x.is_contiguous() and w.is_contiguous() and x.data_ptr() % 8 == 0 and w.data_ptr() % 16 == 0
-            and _lib.use_kernels(x, w)):
+    if (x.is_cuda and 0 < t <= ROUTER_ROWS and t * w.shape[0] <= ROUTER_LOGITS
+            and (t > 1 or w.numel() <= ROUTER_VECTOR) and x.dtype == torch.bfloat16
+            and w.dtype == torch.float32 and h % 4 == 0 and x.is_contiguous() and w.is_contiguous()
+            and x.data_ptr() % 8 == 0 and w.data_ptr() % 16 == 0 and _lib.use_kernels(x, w)):
         out = guard.empty(t, w.shape[0], dtype=torch.float32, device=x.device)
         check(_lib.load().msrl_router_logits(ptr(x), ptr(w), c_int(t), c_int(w.shape[0]), c_int(h), ptr(out), stream()),
               "router_logits")

@@ -257,3 +257,15 @@ def test_router_of_few_tokens(t, e, h, k, norm, factor, biased):
     assert torch.equal(torch.sort(idx, -1).values, torch.sort(want, -1).values)
     p = s.gather(1, idx)
     torch.testing.assert_close(score, (p / p.sum(-1, keepdim=True) if norm else p) * factor, rtol=1e-5, atol=1e-7)
+
+
+@pytest.mark.parametrize("t,e,h,kernel", [(1, 1024, 128, True), (64, 1024, 128, True), (65, 1024, 128, False), (128, 512, 128, True),
+                                          (129, 512, 128, False), (256, 256, 128, True), (257, 8, 128, False),
+                                          (1, 1024, 3072, True), (1, 1024, 3076, False), (2, 1024, 3076, True)])
+def test_router_kernel_only_where_it_was_the_faster_one(t, e, h, kernel):
+    from mindspeed_rl_b200.ops import _lib
+    x, w = torch.randn(t, h, device="cuda").bfloat16(), torch.randn(e, h, device="cuda")
+    before = _lib.launch_count()
+    out = M.router_logits(x, w)
+    assert (_lib.launch_count() > before) == kernel and out.dtype == torch.float32
+    torch.testing.assert_close(out, (x.double() @ w.double().t()).float(), rtol=1e-4, atol=1e-3)
