@@ -484,22 +484,20 @@ delta_scan_kernel(const float* qn, const float* kn, const float* kq, const float
 constexpr int SG = 2;            // groups staged at a time
 
 // The sequence of rank `z` by length.  A block walks its sequence from the first token to the last, so a long one that starts late
-// is what the launch ends with (2048, 1531, 777 and 3001 tokens, 32 heads, in that order: 1289 -> 1083 us).  Beyond 64 sequences
-// there are blocks enough, and finding the rank would cost each of them too much.
+// is what the launch ends with.  Whole calls, 32 heads of 128: 2048, 1531, 777 and 3001 tokens, in that order, 1770 -> 1558 us, 32
+// sequences of 1 to 1400 4015 -> 3870; of one length, 8 of 512 and 32 of 256, 797 and 1505 as before.  Beyond 32, where a lane to a
+// sequence no longer does, there are blocks enough (48 and 64 of uneven length: within 1 %; ranks from shared memory cost every call 2 %).
 __device__ __forceinline__ int longest_first(const int* cu, int z, int n) {
-  if (n == 1 || n > 64) return z;
-  __shared__ int pick;
-  if (threadIdx.x < n) {
-    const int i = threadIdx.x, mine = cu[i + 1] - cu[i];
-    int rank = 0;
-    for (int j = 0; j < n; ++j) {
-      const int other = cu[j + 1] - cu[j];
-      rank += other > mine || (other == mine && j < i);
-    }
-    if (rank == z) pick = i;
+  if (n == 1 || n > 32) return z;
+  const int lane = threadIdx.x & 31, mine = lane < n ? cu[lane + 1] - cu[lane] : -1;     // every warp for itself
+  const int head = __shfl_sync(0xffffffffu, mine, 0);
+  if (__all_sync(0xffffffffu, lane >= n || mine == head)) return z;
+  int rank = 0;
+  for (int j = 0; j < n; ++j) {
+    const int other = __shfl_sync(0xffffffffu, mine, j);
+    rank += other > mine || (other == mine && j < lane);
   }
-  __syncthreads();
-  return pick;
+  return __ffs(__ballot_sync(0xffffffffu, lane < n && rank == z)) - 1;
 }
 
 template <int DPL, int COLS>

@@ -627,3 +627,32 @@ def test_embedding_grad_kernel_matches_fp32_sum(gdtype):
     assert torch.equal(g1, g2)
     tol = 2e-2 if gdtype == torch.bfloat16 else 1e-3
     close(g1.float(), want, tol * want.abs().max().item(), tol, "embedding grad")
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("lens", [[5], [7, 0, 40, 7, 1], [9] * 31, [(13 * i) % 37 for i in range(32)], [(13 * i) % 37 for i in range(33)]])
+def test_delta_prompts_in_any_order_of_lengths(lens, dim):
+    """The longest sequences' blocks start first (up to 32 sequences): every sequence gets the bits that it gets alone, ties, equal
+    lengths and sequences without tokens among them."""
+    from mindspeed_rl_b200.ops.microbench_hybrid import _delta, delta_prefill
+    torch.manual_seed(8)
+    lay, proj, a, gate, w = _delta(sum(lens), heads=2, dim=dim, vdim=dim)
+
+    def run(bounds):
+        n, t0, t1 = len(bounds) - 1, bounds[0], bounds[-1]
+        ring = torch.zeros(n, lay.taps, lay.channels, device=DEV).bfloat16()
+        state = torch.zeros(n, lay.heads, dim, dim, device=DEV)
+        cu = torch.tensor(bounds, dtype=torch.int32, device=DEV) - t0
+        seq = torch.arange(n, dtype=torch.int32, device=DEV).repeat_interleave((cu[1:] - cu[:-1]).long())
+        y = delta_prefill(proj[t0:t1], a[t0:t1], gate[t0:t1], lay, w, ring, state, seq, cu,
+                          torch.zeros(n, dtype=torch.int32, device=DEV), torch.arange(n, device=DEV), 1e-5)
+        return y, state, ring
+
+    bounds = [0] + torch.tensor(lens).cumsum(0).tolist()
+    y, state, ring = run(bounds)
+    for b, n in enumerate(lens):
+        if n:
+            y1, s1, r1 = run(bounds[b:b + 2])
+            assert torch.equal(y[bounds[b]:bounds[b + 1]], y1) and torch.equal(state[b], s1[0]) and torch.equal(ring[b], r1[0])
+        else:
+            assert not state[b].any()
