@@ -244,15 +244,30 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       for (int n = 0; n < n_it && ok; ++n) {
         const int st = n & 1;
         const uint32_t q_addr = base + BWD_X + st * TILE_BYTES, do_addr = base + DKDV_Y + st * TILE_BYTES;
+        // Sixteens of queries that see none of the keys are left out: their P and dS are 0, but 0 times an inf or nan of dO or Q
+        // would reach dV and dK.  Tested once a tile, in front of steps without a branch.
+        const int qr = (i_start + (first + n) % nq) * BM, from = (p.causal ? max(kb - off - qr, 0) : 0) - 15, to = qlen - qr;
+        const bool whole = from <= 0 && to > 112;
+        bool add = n > 0;
         // dV += P^T dO, the first half of each thread's columns as soon as it is there
 #pragma unroll
         for (int part = 0; part < 2; ++part) {
           ok = ok && mbar_wait(&p_part[part], n & 1, p.error, ERR_P);
           if (!ok) break;
           fence_after();
+          if (whole) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            tmem_step(tm_dv, tmem, do_addr, (i >> 1) * 4 + part * 2 + (i & 1), n > 0 || part > 0 || i > 0);
+            for (int i = 0; i < 4; ++i)
+              tmem_step(tm_dv, tmem, do_addr, (i >> 1) * 4 + part * 2 + (i & 1), n > 0 || part > 0 || i > 0);
+          } else {
+#pragma unroll 1
+            for (int i = 0; i < 4; ++i) {
+              const int kk = (i >> 1) * 4 + part * 2 + (i & 1);
+              if (kk * 16 < from || kk * 16 >= to) continue;
+              tmem_step(tm_dv, tmem, do_addr, kk, add);
+              add = true;
+            }
+          }
         }
         if (!ok) break;
         commit(&do_empty[st]);                             // dP of this tile is older
@@ -260,8 +275,15 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         ok = ok && mbar_wait(&ds_ready, n & 1, p.error, ERR_P);
         if (!ok) break;
         fence_after();
+        // dK += dS^T Q
+        if (whole) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) tmem_step(tm_dk, tm_dp, q_addr, kk, n > 0 || kk > 0);   // dK += dS^T Q
+          for (int kk = 0; kk < 8; ++kk) tmem_step(tm_dk, tm_dp, q_addr, kk, n > 0 || kk > 0);
+        } else {
+#pragma unroll 1
+          for (int kk = 0; kk < 8; ++kk)
+            if (kk * 16 >= from && kk * 16 < to) tmem_step(tm_dk, tm_dp, q_addr, kk, n > 0 || kk * 16 >= from + 16);
+        }
         commit(&q_empty[st]);
         if (n + 1 < n_it) dprobs(n + 1);
       }
@@ -513,8 +535,14 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         if (!ok) break;
         fence_after();
         const uint32_t k_addr = base + BWD_X + j % 3 * TILE_BYTES;
+        // dQ += dS K, sixteens of keys that no row sees left out as in dK/dV
+        if (j * 128 + 112 < kmax) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) tmem_step(tm_dq, tmem + (j & 1) * 128, k_addr, kk, j > 0 || kk > 0);   // dQ += dS K
+          for (int kk = 0; kk < 8; ++kk) tmem_step(tm_dq, tmem + (j & 1) * 128, k_addr, kk, j > 0 || kk > 0);
+        } else {
+#pragma unroll 1
+          for (int kk = 0; j * 128 + kk * 16 < kmax; ++kk) tmem_step(tm_dq, tmem + (j & 1) * 128, k_addr, kk, j > 0 || kk > 0);
+        }
         commit(&k_empty[j % 3]);
       }
       if (ok) commit(&done);

@@ -37,16 +37,18 @@ __device__ __forceinline__ float ex2(float x) {
   return d;
 }
 
-// Query tile `item` of KV head hk: row tile item / rep, query head item % rep, and the key tiles [t0, t1) it sees.
+// Query tile `item` of KV head hk: row tile item / rep, query head item % rep, the keys [k0, k1) that its rows see and the key tiles
+// [t0, t1) they lie in.
 struct QueryTile {
-  int m0, h, t0, t1;
+  int m0, h, k0, k1, t0, t1;
   __device__ __forceinline__ QueryTile(const Params& p, int item, int hk, int rep, int qlen, int klen) {
     m0 = item / rep * BM;
     h = hk * rep + item % rep;
     const int off = klen - qlen;
-    const int kmax = p.causal ? min(klen, m0 + BM + off) : klen;
-    t0 = p.window > 0 ? max(m0 + off - p.window + 1, 0) / 128 : 0;
-    t1 = m0 < qlen ? max((max(kmax, 0) + 127) / 128, t0) : t0;
+    k0 = p.window > 0 ? max(m0 + off - p.window + 1, 0) : 0;
+    k1 = max(p.causal ? min(klen, m0 + BM + off) : klen, 0);
+    t0 = k0 / 128;
+    t1 = m0 < qlen ? max((k1 + 127) / 128, t0) : t0;
   }
 };
 
@@ -134,16 +136,28 @@ fa_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       auto pv = [&](int x, int j, const QueryTile& t) {  // O_x += P_x V_j
         const int st = (j - j0) & 1;
         const uint32_t v_addr = base + PAIR_V + st * TILE_BYTES;
+        // Sixteens of keys that no row sees are left out: their P is 0, but 0 times an inf or nan of V would reach the rows.  Tested
+        // once a tile, in front of steps without a branch (a branch a step cost prompts 0.7 to 0.9 %).
+        const int from = t.k0 - j * 128 - 15, to = t.k1 - j * 128;
+        const bool whole = from <= 0 && to > 112;
         ok = mbar_wait(&v_full[st], ((j - j0) >> 1) & 1, p.error, ERR_V);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           ok = ok && mbar_wait(&p_part[x][half], turn[x] & 1, p.error, ERR_P);
           if (!ok) return;
           fence_after();
-#pragma unroll
-          for (int kk = half * 4; kk < half * 4 + 4; ++kk)
+          auto step = [&](int kk, bool add) {
             umma_ts(tmem + 256 + x * 128, tmem + x * 128 + kk * 8, desc_sw128(v_addr + kk * 2048, TILE_HALF, 1024), id_o,
-                    (j > t.t0 || kk > 0) ? 1u : 0u);
+                    add ? 1u : 0u);
+          };
+          if (whole) {
+#pragma unroll
+            for (int kk = half * 4; kk < half * 4 + 4; ++kk) step(kk, j > t.t0 || kk > 0);
+          } else {
+#pragma unroll 1
+            for (int kk = half * 4; kk < half * 4 + 4; ++kk)
+              if (kk * 16 >= from && kk * 16 < to) step(kk, j > t.t0 || kk * 16 >= from + 16);
+          }
         }
         ++turn[x];
       };

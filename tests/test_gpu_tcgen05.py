@@ -340,6 +340,65 @@ def test_flash_attention_bwd_key_tiles(nh, nkv, ql, kl, causal, monkeypatch):
         torch.testing.assert_close(a, c, rtol=2e-2, atol=2e-2 * c.abs().max().item())
 
 
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+@pytest.mark.parametrize("ql,kl,causal,poison", [
+    ([144, 100], [144, 100], True, 144),          # the next sequence from its first row on
+    ([130, 100], [130, 100], True, 144),          # from the next sixteen rows on
+    ([130, 100], [130, 100], False, 144),
+    ([1030, 90, 300] * 3, [1030, 90, 300] * 3, True, 1040),
+    ([200, 40], [264, 140], True, 272),           # more keys than queries
+])
+def test_flash_attention_does_not_read_the_next_sequence(ql, kl, causal, poison, bad):
+    """What follows a sequence in the packed rows takes part in its last tile with weights of exact zeros, which an inf or nan turns
+    into nan: no sixteen rows that lie wholly behind the sequence are multiplied."""
+    from mindspeed_rl_b200 import ops
+    torch.manual_seed(15)
+    nh, nkv = 4, 2
+    cu_q, cu_k = (torch.tensor([0] + list(torch.tensor(x).cumsum(0)), dtype=torch.int32, device=DEV) for x in (ql, kl))
+    q, do = (torch.randn(sum(ql), nh, 128, device=DEV).bfloat16() for _ in range(2))
+    k, v = (torch.randn(sum(kl), nkv, 128, device=DEV).bfloat16() for _ in range(2))
+
+    def run():
+        o, lse = ops.attn_kv_fwd(q, k, v, cu_q, cu_k, max(ql), causal)
+        dq, dk, dv = ops.attn_kv_bwd(do.view(sum(ql), -1), q, k, v, o, lse, cu_q, cu_k, max(ql), max(kl), causal)
+        return o[:ql[0]], lse[:, :ql[0]], dq[:ql[0]], dk[:kl[0]], dv[:kl[0]]
+
+    clean = [x.clone() for x in run()]
+    for x, n in ((q, poison - kl[0] + ql[0]), (do, poison - kl[0] + ql[0]), (k, poison), (v, poison)):
+        x[n:] = bad
+    for a, b in zip(run(), clean):
+        assert bool(a.isfinite().all()) and torch.equal(a, b)
+    G.check_status(torch.device("cuda", torch.cuda.current_device()), "tcgen05 attention")
+
+
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+def test_flash_attention_reads_what_some_row_of_a_tile_sees(bad):
+    """Keys behind the last and before the first that a tile of 128 query rows sees, and queries that see none of 128 keys, do not
+    reach it across a border of sixteen."""
+    from mindspeed_rl_b200 import ops
+    from mindspeed_rl_b200.ops.window import GroupedHeads, window_prefill_attention
+    torch.manual_seed(16)
+    nh, nkv, ql, kl = 4, 2, 200, 264
+    cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device=DEV) for n in (ql, kl))
+    q, do = (torch.randn(ql, nh, 128, device=DEV).bfloat16() for _ in range(2))
+    k, v = (torch.randn(kl, nkv, 128, device=DEV).bfloat16() for _ in range(2))
+    o, lse = ops.attn_kv_fwd(q, k, v, cu_q, cu_k, ql, True)
+    clean = ops.attn_kv_bwd(do.view(ql, -1), q, k, v, o, lse, cu_q, cu_k, ql, kl, True)
+    v2 = v.clone()
+    v2[192:] = bad                                            # row r sees keys up to r + 64: rows 0 to 127 none of these
+    assert torch.equal(ops.attn_kv_fwd(q, k, v2, cu_q, cu_k, ql, True)[0][:128], o[:128])
+    do[:64] = bad                                             # these rows see no key from 128 on
+    for a, b in zip(ops.attn_kv_bwd(do.view(ql, -1), q, k, v, o, lse, cu_q, cu_k, ql, kl, True)[1:], clean[1:]):
+        assert torch.equal(a[128:], b[128:])
+    lay = GroupedHeads(4, 2, 128, 128, 128, 128, 0, 512, 768)
+    t, cu = 500, torch.tensor([0, 500], dtype=torch.int32, device=DEV)
+    proj = torch.randn(t, 1024, device=DEV).bfloat16()
+    want = window_prefill_attention(proj, lay, cu, cu, t, 128 ** -0.5, 150)
+    proj[:96, 768:] = bad                                     # rows from 256 on see keys from 107 on
+    assert torch.equal(window_prefill_attention(proj, lay, cu, cu, t, 128 ** -0.5, 150)[256:], want[256:])
+    G.check_status(torch.device("cuda", torch.cuda.current_device()), "tcgen05 attention")
+
+
 @pytest.mark.parametrize("causal", [False, True])
 def test_block_attention_with_separate_kv(causal):
     """The block primitives of ring attention (queries against a separate K/V block, log-sum-exp of the
