@@ -382,7 +382,7 @@ template <int G>
 __global__ void __launch_bounds__(256)
 headnorm_bwd_kernel(__nv_bfloat16* __restrict__ dy_dx, const __nv_bfloat16* __restrict__ x, HeadLayout L,
                     const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd, float* __restrict__ dw_partial,
-                    unsigned heads, int nheads, int hd) {
+                    long long T, long long chunk, int nheads, int hd) {
   __shared__ float sdw[8][256];    // one row per warp (256 threads): summed in warp order, so that the
                                    // result does not depend on which warp finishes first
   constexpr int U = 2;
@@ -390,43 +390,46 @@ headnorm_bwd_kernel(__nv_bfloat16* __restrict__ dy_dx, const __nv_bfloat16* __re
   const bool act = g * 8 < hd;
   float dw_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, wv[8];
   unpack8(ld8(w + (act ? g * 8 : 0)), wv);
-  for (unsigned base = blockIdx.x * (U * 256 / G); base < heads; base += gridDim.x * (U * 256 / G)) {
-    bf16x8 rd[U], rx[U];
-    long long off[U];
-    float rs[U];
+  for (long long t0 = 0; t0 < T; t0 += chunk, dy_dx += chunk * L.stride_t, x += chunk * L.stride_t, rstd += chunk * nheads) {
+    const unsigned heads = (unsigned)(T - t0 < chunk ? T - t0 : chunk) * (unsigned)nheads;
+    for (unsigned base = blockIdx.x * (U * 256 / G); base < heads; base += gridDim.x * (U * 256 / G)) {
+      bf16x8 rd[U], rx[U];
+      long long off[U];
+      float rs[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const unsigned i = base + u * (256 / G) + threadIdx.x / G, t = i / (unsigned)nheads;
-      off[u] = head_offset(L, t, (int)(i - t * (unsigned)nheads)) + g * 8;
-      rs[u] = 0.f;
-      if (act && i < heads) {
-        rd[u] = ld8(dy_dx + off[u]);
-        rx[u] = ld8(x + off[u]);
-        rs[u] = rstd[i];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const bool on = act && base + u * (256 / G) + threadIdx.x / G < heads;
-      float d[8] = {0, 0, 0, 0, 0, 0, 0, 0}, xv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      float dot = 0.f;
-      if (on) {
-        unpack8(rd[u], d);
-        unpack8(rx[u], xv);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          dw_acc[k] += d[k] * xv[k] * rs[u];
-          d[k] *= wv[k];
-          dot += d[k] * xv[k];
+      for (int u = 0; u < U; ++u) {
+        const unsigned i = base + u * (256 / G) + threadIdx.x / G, t = i / (unsigned)nheads;
+        off[u] = head_offset(L, t, (int)(i - t * (unsigned)nheads)) + g * 8;
+        rs[u] = 0.f;
+        if (act && i < heads) {
+          rd[u] = ld8(dy_dx + off[u]);
+          rx[u] = ld8(x + off[u]);
+          rs[u] = rstd[i];
         }
       }
 #pragma unroll
-      for (int o = G / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-      const float c = dot * rs[u] * rs[u] * rs[u] / (float)hd;
-      if (on) {
+      for (int u = 0; u < U; ++u) {
+        const bool on = act && base + u * (256 / G) + threadIdx.x / G < heads;
+        float d[8] = {0, 0, 0, 0, 0, 0, 0, 0}, xv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        float dot = 0.f;
+        if (on) {
+          unpack8(rd[u], d);
+          unpack8(rx[u], xv);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) d[k] = d[k] * rs[u] - xv[k] * c;
-        st8(dy_dx + off[u], pack8(d));
+          for (int k = 0; k < 8; ++k) {
+            dw_acc[k] += d[k] * xv[k] * rs[u];
+            d[k] *= wv[k];
+            dot += d[k] * xv[k];
+          }
+        }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        const float c = dot * rs[u] * rs[u] * rs[u] / (float)hd;
+        if (on) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) d[k] = d[k] * rs[u] - xv[k] * c;
+          st8(dy_dx + off[u], pack8(d));
+        }
       }
     }
   }
@@ -714,21 +717,27 @@ MSRL_API int msrl_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
   MSRL_LAUNCH_CHECK();
 }
 
+// tokens whose heads count in 32 bits (with room for the last block's)
+static long long head_chunk(int nheads) { return nheads <= 1 ? 1 << 30 : nheads >= (1 << 30) ? 1 : (1 << 30) / nheads; }
+
 MSRL_API int msrl_headnorm_fwd(const void* x, long long stride_t, int group_stride, int hpg,
                                int head_stride, const void* w, void* y, float* rstd, long long T,
                                int nheads, int hd, float eps, cudaStream_t st) {
   if (T == 0) return 0;
   if (hd % 8 != 0 || hd > 256) return (int)cudaErrorInvalidValue;
   HeadLayout L{stride_t, group_stride, hpg, head_stride};
-  const long long heads = T * nheads;
-  if (heads > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
   const int g = hd <= 64 ? 8 : hd <= 128 ? 16 : 32;
-  const int u = heads <= 32LL * sm_count() ? 1 : 4;
+  const int u = T * nheads <= 32LL * sm_count() ? 1 : 4;
   auto* kernel = g == 8    ? (u == 1 ? headnorm_fwd_kernel<8, 1> : headnorm_fwd_kernel<8, 4>)
                  : g == 16 ? (u == 1 ? headnorm_fwd_kernel<16, 1> : headnorm_fwd_kernel<16, 4>)
                            : (u == 1 ? headnorm_fwd_kernel<32, 1> : headnorm_fwd_kernel<32, 4>);
-  kernel<<<(unsigned)ceil_div(heads, u * 256 / g), 256, 0, st>>>((const __nv_bfloat16*)x, L, (const __nv_bfloat16*)w,
-                                                                 (__nv_bfloat16*)y, rstd, (unsigned)heads, nheads, hd, eps);
+  const long long chunk = head_chunk(nheads);
+  for (long long t0 = 0; t0 < T; t0 += chunk) {
+    const unsigned heads = (unsigned)(T - t0 < chunk ? T - t0 : chunk) * (unsigned)nheads;
+    kernel<<<(unsigned)ceil_div(heads, u * 256 / g), 256, 0, st>>>(
+        (const __nv_bfloat16*)x + t0 * stride_t, L, (const __nv_bfloat16*)w, (__nv_bfloat16*)y + t0 * stride_t,
+        rstd != nullptr ? rstd + t0 * nheads : nullptr, heads, nheads, hd, eps);
+  }
   MSRL_LAUNCH_CHECK();
 }
 
@@ -742,11 +751,9 @@ MSRL_API int msrl_headnorm_bwd(void* dy_dx, const void* x, long long stride_t, i
   if (hd % 8 != 0 || hd > 256) return (int)cudaErrorInvalidValue;
   HeadLayout L{stride_t, group_stride, hpg, head_stride};
   const int nb = msrl_headnorm_bwd_blocks();
-  const long long heads = T * nheads;
-  if (heads > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
   auto* kernel = hd <= 64 ? headnorm_bwd_kernel<8> : hd <= 128 ? headnorm_bwd_kernel<16> : headnorm_bwd_kernel<32>;
   kernel<<<nb, 256, 0, st>>>((__nv_bfloat16*)dy_dx, (const __nv_bfloat16*)x, L, (const __nv_bfloat16*)w, rstd, dw_partial,
-                             (unsigned)heads, nheads, hd);
+                             T, head_chunk(nheads), nheads, hd);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   colsum_partials_kernel<<<(hd + 31) / 32, COLSUM_WARPS * 32, 0, st>>>(dw_partial, nb, hd, dw_f32,

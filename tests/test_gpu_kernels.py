@@ -123,6 +123,27 @@ def test_headnorm_and_rope_sizes(hd, t, nh, nkv):
     close(a, b, 4e-2, 2e-2, "rope")
 
 
+def test_headnorm_of_more_heads_than_31_bits_count():
+    """2049 tokens of 2^20 heads of 8 that all lie in the same place, forward and backward (of a gradient that the norm hands on as it
+    is: orthogonal to ones, unit weights and scales)."""
+    from mindspeed_rl_b200.ops._lib import c_float, c_int, c_ll, check, ptr, stream
+    from mindspeed_rl_b200.ops.elementwise import _workspace
+    torch.manual_seed(5)
+    n, t, hd, lib = 1 << 20, 2049, 8, _lib.load()
+    x, y = torch.randn(n, hd, device=DEV).bfloat16(), torch.zeros(n, hd, device=DEV).bfloat16()
+    w = torch.ones(hd, device=DEV).bfloat16()
+    where = (c_ll(0), c_int(0), c_int(n), c_int(hd))
+    check(lib.msrl_headnorm_fwd(ptr(x), *where, ptr(w), ptr(y), None, c_ll(t), c_int(n), c_int(hd), c_float(1e-6), stream()), "fwd")
+    close(y, (x.float() * torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + 1e-6)).bfloat16(), 1e-2, 1e-2, "headnorm")
+    sign = torch.tensor([1.0, -1.0], device=DEV).repeat(hd // 2)
+    dy, ones, rstd, dw = sign.bfloat16().repeat(n, 1), torch.ones_like(x), torch.ones(t * n, device=DEV), torch.zeros(hd, device=DEV)
+    part = _workspace("headnorm_dw", lib.msrl_headnorm_bwd_blocks() * hd, x.device)
+    check(lib.msrl_headnorm_bwd(ptr(dy), ptr(ones), *where, ptr(w), ptr(rstd), ptr(part), ptr(dw), None, c_int(1), c_ll(t), c_int(n),
+                                c_int(hd), stream()), "bwd")
+    assert torch.equal(dy.float(), sign.repeat(n, 1))
+    torch.testing.assert_close(dw, sign * (t * n), rtol=1e-6, atol=0)
+
+
 @pytest.mark.parametrize("t", [1, 3, 257])
 @pytest.mark.parametrize("nh,nkv,hd", [(32, 4, 128), (32, 8, 128), (5, 1, 256), (3, 3, 24)])
 def test_rope_head_counts(nh, nkv, hd, t):
