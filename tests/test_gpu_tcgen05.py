@@ -278,6 +278,35 @@ def test_flash_attention_fwd_query_tile_pairs(nh, nkv, ql, kl, causal, monkeypat
         torch.testing.assert_close(lse.cpu(), lse_r, rtol=1e-4, atol=1e-3)
 
 
+@pytest.mark.parametrize("window", [1, 65, 128, 129, 300, None])
+@pytest.mark.parametrize("nh,nkv,form", [(4, 4, "plain"), (6, 2, "plain"), (4, 4, "all"), (6, 2, "all"), (6, 2, "cap"), (6, 2, "sink"),
+                                         (4, 4, "gate")])
+def test_flash_attention_fwd_pairs_with_windows_and_score_forms(nh, nkv, form, window):
+    """Two query tiles to a block whose key ranges start and end at different tiles (every pair crosses row tiles without groups,
+    some do with three heads to a group), soft caps, sinks and gates, more keys than queries; against the fp32 formulation."""
+    from mindspeed_rl_b200 import ops
+    from mindspeed_rl_b200.ops.window import GroupedHeads, window_prefill_attention
+    torch.manual_seed(17)
+    ql, more = [700, 1, 127, 129, 385, 640, 250], [0, 300, 1, 77, 128, 200, 515]
+    kl = [a + b for a, b in zip(ql, more)]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert (max(ql) + 127) // 128 * nh * len(ql) > sms            # below that a block takes one query tile
+    cu_q, cu_k = (torch.tensor([0] + list(torch.tensor(x).cumsum(0)), dtype=torch.int32, device=DEV) for x in (ql, kl))
+    lay = GroupedHeads(nh, nkv, 128, 128, 128, 128, 0, nh * 128, (nh + nkv) * 128)
+    proj = (4.0 * torch.randn(sum(ql), (nh + 2 * nkv) * 128, device=DEV)).bfloat16()
+    k, v = (torch.randn(sum(kl), nkv, 128, device=DEV).bfloat16() for _ in range(2))
+    f = ops.ScoreForm(softcap=6.0 if form in ("cap", "all") else 0.0,
+                      gate=torch.randn(sum(ql), nh, device=DEV).bfloat16() if form in ("gate", "all") else None,
+                      sink=2.0 * torch.randn(nh, device=DEV) if form in ("sink", "all") else None)
+    got = window_prefill_attention(proj, lay, cu_q, cu_k, max(ql), 128 ** -0.5, window, kv=(k, v), form=f)
+    G.check_status(torch.device("cuda", torch.cuda.current_device()), "tcgen05 attention")
+    host = ops.ScoreForm(f.softcap, *(None if x is None else x.cpu() for x in (f.gate, f.sink)))
+    want = window_prefill_attention(proj.cpu(), lay, cu_q.cpu(), cu_k.cpu(), max(ql), 128 ** -0.5, window, kv=(k.cpu(), v.cpu()),
+                                    form=host)
+    # P and the output are rounded to bf16 (2^-9 each) over values of order one
+    torch.testing.assert_close(got.float().cpu(), want.float(), rtol=2e-2, atol=2e-2)
+
+
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("nh,nkv,interleaved", [(4, 2, True), (7, 1, False)])
 def test_flash_attention_bwd_tcgen05(nh, nkv, interleaved, causal, monkeypatch):
