@@ -19,8 +19,8 @@
 namespace msrl {
 namespace fa5 {
 
-constexpr int BWD_WARPS = 8, BWD_TMA = 8, BWD_MMA = 9, BWD_THREADS = 384;      // warps 0-7 soft-max, 8 TMA, 9 MMA
-constexpr int NC = 512 / BWD_WARPS;                    // columns of a soft-max thread
+constexpr int BWD_WARPS = 8, BWD_TMA = 8, BWD_MMA = 9, BWD_THREADS = 320;      // warps 0-7 soft-max, 8 TMA, 9 MMA
+constexpr int NC = 64;                                 // columns of a soft-max thread: 128 over two warpgroups
 // Two resident tiles (K, V or Q, dO) and stages of the two that stream by.
 constexpr uint32_t BWD_A = 0, BWD_B = TILE_BYTES, BWD_X = 2 * TILE_BYTES, DKDV_Y = 4 * TILE_BYTES, DKDV_SMEM = 6 * TILE_BYTES;
 // dQ: three stages of K, which the last product of a step frees and the next but one step reads first (with two, every step waited
@@ -123,13 +123,13 @@ __device__ __forceinline__ uint32_t pack_bf16(float2 v) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// SPLIT: blocks of one cluster share a key tile, each with a contiguous part of its (query head, query tile) list; their dK and
-// dV meet in shared memory at the end, added in rank order.
-template <bool SPLIT>
+// SPLITS blocks of one cluster (or one block alone) share a key tile, each with a contiguous part of its (query head, query tile)
+// list; their dK and dV meet in shared memory at the end, added in rank order.
+template <int SPLITS>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                    const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                   const __grid_constant__ BwdParams p, const int splits) {
+                   const __grid_constant__ BwdParams p) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -137,7 +137,7 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   __shared__ uint32_t tmem_slot;
   __shared__ __align__(16) float stat[2][2][128];        // per stage: -lse (exp2 domain) and -delta of its query rows
 
-  const int rank = SPLIT ? blockIdx.x % splits : 0, work = SPLIT ? blockIdx.x / splits : blockIdx.x;
+  const int rank = blockIdx.x % SPLITS, work = blockIdx.x / SPLITS;
   const int hk = work % p.nkv, b = work / p.nkv % p.batch, kb = work / p.nkv / p.batch * BM;   // first key of this block
   const int q0 = p.cu_q[b], qlen = p.cu_q[b + 1] - q0;
   const int k0 = p.cu_k[b], klen = p.cu_k[b + 1] - k0;
@@ -146,8 +146,7 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   // query tiles that see any of these keys: rows r with r + off >= kb (causal), r < qlen
   const int i_start = p.causal ? max(0, kb - off) / BM : 0;
   const int nq = max(0, (qlen + BM - 1) / BM - i_start), all = nq * rep;
-  const int first = SPLIT ? (int)((long long)all * rank / splits) : 0;
-  const int n_it = (SPLIT ? (int)((long long)all * (rank + 1) / splits) : all) - first;
+  const int first = (int)((long long)all * rank / SPLITS), n_it = (int)((long long)all * (rank + 1) / SPLITS) - first;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -362,7 +361,7 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     if (ok && n_it > 0) fence_after();
     const int kc = head_col(0, p.k_group_stride, p.k_hpg, p.k_head_stride, hk);
     const int vc = head_col(0, p.v_group_stride, p.v_hpg, p.v_head_stride, hk);
-    if constexpr (!SPLIT) {
+    if constexpr (SPLITS == 1) {
       if (ok) {
         unsigned char* patch = smem + warp * (32 * OUT_PITCH);
         const int rows_valid = klen - (kb + quarter * 32);
@@ -394,17 +393,18 @@ fa_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       }
     }
   }
-  if constexpr (SPLIT) {
+  if constexpr (SPLITS > 1) {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     // rank r adds up and stores its share of the rows; 16 threads to a row, 8 columns each
-    const int per = BM / splits, col = threadIdx.x & 15;
+    constexpr int per = BM / SPLITS;
+    const int col = threadIdx.x & 15;
     const uint32_t base = smem_u32(smem);
     for (int i = threadIdx.x >> 4; i < 2 * per; i += BWD_THREADS / 16) {
       const int which = i / per, row = rank * per + i % per;
       if (kb + row >= klen) continue;
       float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int r = 0; r < splits; ++r) {
+      for (int r = 0; r < SPLITS; ++r) {
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t at;
@@ -600,7 +600,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (lane == 0) mbar_arrive(&ds_ready);
     }
     if (ok && n_tiles > 0) ok = mbar_wait_warp(&done, 0, p.error, ERR_PV);
-    if (ok && wg < 2) {
+    if (ok) {
       if (n_tiles > 0) fence_after();
       const int qc = head_col(0, p.q_group_stride, p.q_hpg, p.q_head_stride, h);
       store_half_tile(tm_dq + lanes + wg * 64, p.scale, n_tiles == 0, smem + warp * (32 * OUT_PITCH), lane,

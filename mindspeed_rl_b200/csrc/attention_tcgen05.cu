@@ -190,8 +190,8 @@ fa_fwd_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     }
   } else {
     // ---------------- soft-max + epilogue ----------------
-    // Two threads per query row: warps 0-3 own key columns [0, 64) of the tile, warps 4-7 columns
-    // [64, 128) (a warp reaches the TMEM lanes of its quarter, warp % 4).  Both read the whole
+    // Two threads per query row: warps 0-3 own key columns [0, 32) of the tile, warps 4-7 columns
+    // [32, 64) (a warp reaches the TMEM lanes of its quarter, warp % 4).  Both read the whole
     // score row for its maximum, so they agree on the running maximum without talking; each keeps
     // the partial sum of its own columns, rescales its half of the O columns and writes its half
     // of P.
@@ -535,7 +535,7 @@ MSRL_API int msrl_flash_attn_varlen_bwd_tcgen05(const void* q, const void* k, co
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(fa5::fa_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dq);
-    for (auto* kernel : {fa5::fa_bwd_dkdv_kernel<false>, fa5::fa_bwd_dkdv_kernel<true>})
+    for (auto* kernel : {fa5::fa_bwd_dkdv_kernel<1>, fa5::fa_bwd_dkdv_kernel<2>})
       if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_kv);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
@@ -553,7 +553,7 @@ MSRL_API int msrl_flash_attn_varlen_bwd_tcgen05(const void* q, const void* k, co
   const long long warps = Tq * nh;
   fa5::fa_delta128_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(p);
   if (splits == 1) {
-    fa5::fa_bwd_dkdv_kernel<false><<<(unsigned)kv_blocks, fa5::BWD_THREADS, smem_kv, st>>>(mq, mdo, mk, mv, p, 1);
+    fa5::fa_bwd_dkdv_kernel<1><<<(unsigned)kv_blocks, fa5::BWD_THREADS, smem_kv, st>>>(mq, mdo, mk, mv, p);
   } else {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(kv_blocks * splits));
@@ -566,7 +566,7 @@ MSRL_API int msrl_flash_attn_varlen_bwd_tcgen05(const void* q, const void* k, co
     cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
     cfg.attrs = &cluster;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, fa5::fa_bwd_dkdv_kernel<true>, mq, mdo, mk, mv, p, splits);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fa5::fa_bwd_dkdv_kernel<2>, mq, mdo, mk, mv, p);
     if (e != cudaSuccess) return (int)e;
   }
   fa5::fa_bwd_dq_kernel<<<(unsigned)q_blocks, fa5::BWD_THREADS, smem_dq, st>>>(mq, mdo, mk, mv, p, (int)q_tiles);

@@ -34,6 +34,8 @@ __device__ __forceinline__ bf16x8 ld8(const __nv_bfloat16* p) {
 __device__ __forceinline__ void st8(__nv_bfloat16* p, const bf16x8& x) {
   *reinterpret_cast<bf16x8*>(p) = x;
 }
+// silu(g) * u: one expression for the SwiGLU kernel and the GEMM epilogues that stand in for it bit by bit
+__device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.f + __expf(-g)) * u; }
 __device__ __forceinline__ void unpack8(const bf16x8& x, float* f) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {

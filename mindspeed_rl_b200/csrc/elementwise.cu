@@ -527,7 +527,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ in,
     unpack8(ld8(in + t * 2 * F + i * 8), g);
     unpack8(ld8(in + t * 2 * F + F + i * 8), u);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = g[k] / (1.f + __expf(-g[k])) * u[k];
+    for (int k = 0; k < 8; ++k) o[k] = silu_mul(g[k], u[k]);
     st8(out + t * F + i * 8, pack8(o));
   }
 }

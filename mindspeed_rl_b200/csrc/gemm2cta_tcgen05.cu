@@ -493,7 +493,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             for (int j = 0; j < 32; ++j) {
               // both products rounded to bf16 first, as when they go through memory
               const float gg = __bfloat162float(__float2bfloat16(g[j])), uu = __bfloat162float(__float2bfloat16(u[j]));
-              g[j] = gg / (1.f + __expf(-gg)) * uu;
+              g[j] = silu_mul(gg, uu);
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q)

@@ -189,7 +189,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
               const float gg = __bfloat162float(__float2bfloat16(v[j])), uu = __bfloat162float(__float2bfloat16(u[j]));
-              v[j] = gg / (1.f + __expf(-gg)) * uu;
+              v[j] = silu_mul(gg, uu);
             }
           }
 #pragma unroll
