@@ -124,6 +124,20 @@ def test_gemm_pair_swiglu(m, f, k):
         _assert_close(got, torch.nn.functional.silu(gate_up[:, :f].float()) * gate_up[:, f:].float(), k)
 
 
+@pytest.mark.parametrize("m,f,k,keep,launches", [(300, 6144, 896, False, 1), (300, 6144, 896, True, 2), (300, 6144, 1536, True, 1),
+                                                 (256, 6144, 1536, True, 2), (256, 6144, 1536, False, 1)])
+def test_linear_swiglu_in_one_kernel_where_it_is_the_faster_one(m, f, k, keep, launches):
+    torch.manual_seed(4)
+    x, w = torch.randn(m, k, device=DEV).bfloat16(), (k ** -0.5 * torch.randn(2 * f, k, device=DEV)).bfloat16()
+    before = _lib.launch_count()
+    act, gate_up = G.linear_swiglu(x, w, keep)
+    assert _lib.launch_count() - before == launches and (gate_up is not None) == keep
+    both = G.gemm_pair(x, w)
+    assert not keep or torch.equal(gate_up, both)
+    _assert_close(act, torch.nn.functional.silu(both[:, :f].float()) * both[:, f:].float(), 16)
+    G.check_status(DEV)
+
+
 @pytest.mark.parametrize("m", [1, 127, 128, 129, 256, 257, 300, 384, 385, 1409])
 @pytest.mark.parametrize("v,k", [(1000, 264), (2500, 1800)])
 def test_lmhead_stats_forms(m, v, k):
