@@ -92,6 +92,13 @@ def route_top(logits: torch.Tensor, top: int, chosen_softmax: bool = False) -> T
     return idx[:, :top].contiguous(), torch.softmax(z, dim=-1) if chosen_softmax else torch.sigmoid(z)
 
 
+def softmax_top_pays(experts: int, top: int) -> bool:
+    """Whether the kernel of :func:`route_softmax_top` is the way for a choice that torch's soft-max, top-k and gather give as well: it
+    takes 1024 router outputs, one pass over them for each expert chosen.  Kernel / torch, us: 128 experts, top 8, the kernel by far;
+    1024, top 32, 48 tokens 25 / 48, 16384 211 / 518; 512, top 128, 48 tokens 68 / 44, 16384 746 / 478."""
+    return experts <= 1024 and top <= 32
+
+
 def route_softmax_top(logits: torch.Tensor, correction: Optional[torch.Tensor], top: int, norm: bool = False,
                       factor: float = 1.0) -> Tuple[torch.Tensor, torch.Tensor]:
     """Router logits ``[T, E]`` fp32 -> ``(ids [T, top] int64, scores [T, top] fp32)``: the ``top`` largest of

@@ -54,7 +54,7 @@ class MoEWeights:
         cfg = self.cfg
         logits = K.router_logits(x, self.router_w)
         if (cfg.moe_router_score_function == "sigmoid" or (cfg.moe_router_num_groups and cfg.moe_router_group_topk)
-                or not logits.is_cuda or logits.shape[1] > 1024):
+                or not logits.is_cuda or not K.softmax_top_pays(logits.shape[1], cfg.moe_router_topk)):
             return route(logits, cfg, self.expert_bias)[:2]
         bias = None if self.expert_bias is None else self.expert_bias.float().contiguous()
         idx, score = K.route_softmax_top(logits, bias, cfg.moe_router_topk, bool(cfg.norm_topk_prob),

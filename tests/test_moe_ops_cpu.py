@@ -73,3 +73,9 @@ def test_route_softmax_top_asks_for_the_correction_on_the_device_too(monkeypatch
     assert any(x is correction for x in asked[0])
     idx, score = M.route_softmax_top(logits, None, 2)
     assert torch.equal(idx, logits.topk(2).indices) and score.shape == (5, 2)
+
+
+def test_router_choice_kernel_only_for_few_chosen_experts():
+    """One pass over the router's outputs for each expert chosen: torch's top-k where many are."""
+    assert M.softmax_top_pays(128, 8) and M.softmax_top_pays(1024, 32)
+    assert not M.softmax_top_pays(1025, 8) and not M.softmax_top_pays(512, 33)
