@@ -204,8 +204,10 @@ rmsnorm_fwd_regs_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 // while keeping partial sums of dw = sum_rows dy * x * rstd in registers; the partials go to
 // `dw_partial[gridDim.x, H]` (scratch) and stage 2 reduces them over blocks.
 // The loads of the next row are in flight while a row is summed, and one barrier a row is enough; bound by reading dy, x (and dres)
-// and writing dx once.  Against loads in the row's turn and two barriers, 32768 x 3584 with dres: 511 -> 182 us (5.2 TB/s),
-// 8416 x 3584 139 -> 52, 1481 x 4096 29.9 -> 14.3.
+// and writing dx once.  Whole calls (with stage 2) from cold caches against loads in the row's turn and two barriers, with dres:
+// 32768 x 3584 376 -> 196 us, 8416 x 3584 116 -> 65, 1481 x 4096 44 -> 28.  Above 4096 columns the prefetch takes 201 to 249 registers
+// and one block of 256 threads an SM is resident where two were; the loads in flight are worth more: 32768 x 5120 513 -> 312, 32768 x
+// 7168 663 -> 433, 1481 x 5120 48 -> 34, 1481 x 8192 65 -> 48, 16 x 7168 17.4 -> 15.4.
 template <int THREADS, int VPT>
 __global__ void __launch_bounds__(THREADS)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
@@ -686,7 +688,8 @@ MSRL_API int msrl_rmsnorm_fwd(const void* x, const void* res, const void* w, voi
 
 // Number of blocks (= rows of the dw scratch) the backward uses for a given problem.
 MSRL_API int msrl_rmsnorm_bwd_blocks(long long rows) {
-  // two blocks to an SM: one 281 us for 32768 x 3584, two 182, three 233, four 186 (the partial sums cost cap x H floats)
+  // two blocks to an SM, kernel alone, 32768 x 3584: one 281 us, two 182, three 233, four 186 (the partial sums cost cap x H floats);
+  // above 4096 columns one of the two is resident at a time, which is still the faster form (see the kernel)
   long long cap = (long long)sm_count() * 2;
   return (int)(rows < cap ? (rows < 1 ? 1 : rows) : cap);
 }

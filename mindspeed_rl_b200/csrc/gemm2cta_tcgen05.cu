@@ -838,8 +838,8 @@ MSRL_API int msrl_lmhead_stats_tiles(int N) { return (N + g2::BN - 1) / g2::BN; 
 
 // LM head fused with the log-softmax statistics: stats[column tile, M] records over 256-column tiles of z = (H W^T) * inv_temp;
 // combine them with msrl_logprob_finish(nshard = tiles * shards).  On CTA pairs, which pull half as much of W through L2 and
-// shared memory as a block alone (128 x 256 tiles before): 16384 tokens, 152064 x 3584: 16038 -> 12932 us (1381 TFLOP/s).  Where
-// the last 256 rows are at most half full, or the inner size is small, the caller takes the form with row tiles of 128
+// shared memory as a block alone (128 x 256 tiles before); 152064 x 3584, single CTAs / pairs in turn: 4096 tokens 2799 / 2702 us,
+// 16384 16649 / 14765, 32768 35144 / 31330, all at the clock that the power limit leaves.  Where the last 256 rows are at most half full, or the inner size is small, the caller takes the form with row tiles of 128
 // (gemm_tcgen05.cu).
 MSRL_API int msrl_lmhead_stats(const void* H, long long ldh, const void* W, long long ldw, const long long* labels,
                                int vocab_offset, float inv_temp, void* stats, int M, int N, int K, int* error,
